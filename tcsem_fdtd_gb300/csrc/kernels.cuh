@@ -99,17 +99,20 @@ void launch_update_e(const Geom &g, FieldSet<T> f, const T *con, const Axis<T> &
                      const SourceTable<T> &src, int *err, cudaStream_t st);
 template <typename T>
 void launch_bderivate(const Geom &g, FieldSet<T> f, const Axis<T> &ax, T dtb, int *err, cudaStream_t st);
-// TMA descriptors of the fused sweep's inputs: ex ey ez bx by bz of one field set, then sigma
+// TMA descriptors of one sweep: its inputs ex ey ez bx by bz of one field set, then sigma (the padded
+// arrays, boxes with halo), and its outputs ex ey ez bx by bz of the other set (the cells i < L, j < M,
+// k < N, boxes of one tile)
 struct SweepMaps {
     CUtensorMap m[7];
+    CUtensorMap o[6];
 };
 // chunks c0 .. c1-1 in one launch; rev = the last chunk's blocks first (consecutive
 // steps alternate, so a step starts on the planes the previous one wrote last,
 // which may still be in L2); pdl = programmatic dependent launch after the previous
 // kernel on the stream (the CTAs wait for it before loading the air plane k = -1)
 template <typename T>
-void launch_fused_sweep(const SweepMaps &maps, const Geom &g, FieldSet<T> out, const T *tin, T *tout,
-                        const Axis<T> &ax, StepScalars<T> s, const StepScalars<T> *table, StepGate gate,
+void launch_fused_sweep(const SweepMaps &maps, const Geom &g, const T *tin, T *tout, const Axis<T> &ax,
+                        StepScalars<T> s, const StepScalars<T> *table, StepGate gate,
                         const SourceTable<T> &src, const ZChunks &zc, int c0, int c1, bool rev, int *err,
                         cudaStream_t st, bool pdl = false);
 template <typename T> cudaError_t sweep_configure(int N);
@@ -117,6 +120,8 @@ template <typename T> size_t sweep_smem_bytes(int N);
 template <typename T> int sweep_blocks_per_sm(int N);  // resident sweep CTAs per SM (after sweep_configure)
 int sweep_box_x();
 int sweep_box_y();
+int sweep_tile_x();
+int sweep_tile_y();
 template <typename T> void launch_bz_consolidate(const Geom &g, T *bz, T *tot, const ZChunks &zc, cudaStream_t st);
 
 // ------------------------------------------------------------------ batches
@@ -142,7 +147,6 @@ struct BatchIndex {
 template <typename T> struct SweepSlot {
     SweepMaps maps;
     Geom g;
-    FieldSet<T> out;
     const T *tin;
     T *tout;
     Axis<T> ax;

@@ -128,7 +128,7 @@ template <typename T> __device__ int run_item(const PersistArgs<T> &a, const int
         const long st = (long)*d.step_base + step;
         if (st >= d.nsteps) return 0;
         const int bx = u % d.tiles_x, rest = u / d.tiles_x, by = rest % d.tiles_y, c = rest / d.tiles_y;
-        sweep_cta<T, true>(d.maps, d.g, d.out, d.tin, d.tout, d.ax, d.table[st], d.src, d.zc, bx, by, c, d.err);
+        sweep_cta<T, true>(d.maps, d.g, d.tin, d.tout, d.ax, d.table[st], d.src, d.zc, bx, by, c, d.err);
         return 2;
     }
     default: {

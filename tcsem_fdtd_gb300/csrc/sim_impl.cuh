@@ -174,7 +174,7 @@ template <typename T> struct SimImpl : SimBase {
     Geom g{};
     DevMem fld[2][6], con, tot[2];  // two field sets + conductivity; per-set chunk totals of Bz
     ZChunks zc{};
-    SweepMaps maps[2];              // TMA descriptors of each field set (+ conductivity)
+    SweepMaps maps[2];              // TMA descriptors of the sweep that reads each field set
     DevMem errw;                    // device error word (a bounded wait gave up)
     DevMem axis_mem;
     Axis<T> ax{};
@@ -437,15 +437,20 @@ template <typename T> struct SimImpl : SimBase {
         const cuuint32_t box[3] = {(cuuint32_t)sweep_box_x(), (cuuint32_t)sweep_box_y(), 1};
         const cuuint32_t estr[3] = {1, 1, 1};
         const CUtensorMapDataType dt = sizeof(T) == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
-        auto make = [&](void *ptr, CUtensorMap *m) {
-            CUresult r = enc(m, dt, 3, ptr, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+        const cuuint64_t odims[3] = {(cuuint64_t)g.L, (cuuint64_t)g.M, (cuuint64_t)g.N};
+        const cuuint32_t obox[3] = {(cuuint32_t)sweep_tile_x(), (cuuint32_t)sweep_tile_y(), 1};
+        auto make = [&](void *ptr, CUtensorMap *m, const cuuint64_t *dim, const cuuint32_t *bx) {
+            CUresult r = enc(m, dt, 3, ptr, dim, strides, bx, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                              CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
             if (r != CUDA_SUCCESS) throw Error(TCSEM_ERR_CUDA, "cuTensorMapEncodeTiled failed (" + std::to_string((int)r) + ")");
         };
         for (int b = 0; b < 2; b++) {
-            for (int a = 0; a < 6; a++) make(fld[b][a].p, &maps[b].m[a]);
-            make(con.p, &maps[b].m[6]);
+            for (int a = 0; a < 6; a++) {
+                make(fld[b][a].p, &maps[b].m[a], dims, box);
+                make(fld[b ^ 1][a].as<T>() + g.at(0, 0, 0), &maps[b].o[a], odims, obox);
+            }
+            make(con.p, &maps[b].m[6], dims, box);
         }
         errw.alloc(sizeof(int));
         dev_bytes += sizeof(int);
@@ -472,7 +477,7 @@ template <typename T> struct SimImpl : SimBase {
         // the others leaves free instead of delaying them (measured: 119.0 µs for the whole
         // 256 x 256 x 160 sweep against 121.8 alternating and 125.4 with the top chunk first)
         const bool short_top = c0 == 0 && c1 - c0 > 1 && zc.kb[1] - zc.kb[0] < zc.kb[2] - zc.kb[1];
-        launch_fused_sweep<T>(maps[b], g, fs(b ^ 1), tot[b].as<T>(), tot[b ^ 1].as<T>(), ax, s, table, gate, src, zc,
+        launch_fused_sweep<T>(maps[b], g, tot[b].as<T>(), tot[b ^ 1].as<T>(), ax, s, table, gate, src, zc,
                               c0, c1, short_top || (b & 1) != 0, errw.as<int>(), st ? st : stream, pdl);
     }
     void consolidate(int b) { launch_bz_consolidate<T>(g, fs(b).bz, tot[b].as<T>(), zc, stream); }
@@ -836,7 +841,7 @@ template <typename T> struct SimImpl : SimBase {
     // ---- batches: the descriptors of one step that reads field set b and writes b ^ 1
     void batch_slot(int b, const int *counter, SweepSlot<T> &sw, BoundarySlot<T> &bs, RxSlot<T> &rs) {
         FieldSet<T> in = fs(b), out = fs(b ^ 1);
-        sw.maps = maps[b]; sw.g = g; sw.out = out; sw.tin = tot[b].as<T>(); sw.tout = tot[b ^ 1].as<T>();
+        sw.maps = maps[b]; sw.g = g; sw.tin = tot[b].as<T>(); sw.tout = tot[b ^ 1].as<T>();
         sw.ax = ax; sw.table = steps.as<StepScalars<T>>(); sw.step_base = counter; sw.nsteps = sched.nsteps;
         sw.src = src; sw.zc = zc; sw.err = errw.as<int>();
         sw.tiles_x = sweep_tiles_x(g.L); sw.tiles_y = sweep_tiles_y(g.M);

@@ -4,6 +4,7 @@
 #include "async.cuh"
 #include "check.cuh"
 #include "kernels.cuh"
+#include "pair.cuh"
 
 namespace tcsem {
 
@@ -11,25 +12,35 @@ namespace tcsem {
 //
 // One pass per time step over the volume: old E/B/sigma planes stream into a
 // shared-memory ring through TMA bulk-tensor copies (cp.async.bulk.tensor,
-// mbarrier completion), the new E and B go to the other buffer of the
-// ping-pong pair.  Tiles are 64 x 8 columns, aligned so every TMA box starts
-// on a 16-byte boundary; each thread owns two columns of a row (x = lane and
-// lane + 32) and marches them z bottom-up through one
-// z-chunk.  Warps 0..7 own the tile rows, warp 8 recomputes the +y halo row
-// and warp 9 the +x halo column (E and the B components the tile's Bz needs),
-// so no CTA waits for another; the -x/-y halo is plain old data in the TMA box.
-// Neighbour values of the new fields go through double-buffered shared planes
-// with one __syncthreads per z-plane:
-//   iteration k:  B(k+1)  ->  E(k)  ->  publish Ez(k), B(k+1)  ->  sync
-//                 ->  TMA of plane k-4 into the freed slot  ->  Bz(k+1)
+// mbarrier completion): stage k of the ring is what the iteration of plane k reads,
+// E and Bz of plane k and Bx, By and sigma of plane k-1 (those of plane k are in
+// registers from the iteration before), so a slot is free after its iteration
+// and every copy has three iterations to arrive.  The new E and B go to the other buffer of the
+// ping-pong pair through shared-memory planes that the TMA stores.  Tiles are
+// 64 x 8 columns, aligned so every TMA box starts on a 16-byte boundary; each
+// thread owns two columns of a row (x = lane and lane + 32) and marches them z
+// bottom-up through one z-chunk, the two cells side by side in packed FP32
+// arithmetic (pair.cuh).  Warps 0..7 own the tile rows, warp 8 recomputes the +y
+// halo row and warp 9 the +x halo column (E and the B components the tile's Bz
+// needs), so no CTA waits for another; the -x/-y halo is plain old data in the
+// TMA box.  Neighbour values of the new fields go through the same shared
+// planes that are stored, double-buffered, with one __syncthreads per z-plane:
+//   iteration k:  B(k+1)  ->  E(k)  ->  publish E(k), B(k+1)  ->  sync
+//                 ->  TMA store of E(k), B(k+1), Bz(k+2); TMA load of stage k-4 into the freed slot
+//                 ->  Bz(k+1)
+//
+// What bounds it: memory.  256 x 256 x 160 in FP32 (545 MB of algorithmic traffic, 80 us at the copy rate)
+// takes 111.1 us, with DRAM busy 69 % of the time and issue slots 40 %; with register stores, scalar
+// arithmetic and two iterations of lead for the copies it was 119.3 us and 74 instead of 49 million
+// warp-instructions.  The pieces, measured one after the other: TMA stores and packed arithmetic 115.8 us
+// (and 17 -> 14.5 us on 64 x 64 x 48, which stays in L2), the third iteration of lead 111.1 us.
 //
 // Bz within a chunk is the partial sum P(k) = sum_{k'=k}^{k1-1} dz div_xy B(k');
 // the true Bz(k) = P(k) + O_c with O_c = sum of the chunk totals T_c' of the
 // chunks below (c' > c).  Readers add O_c; T has one plane per chunk.
 
 namespace fs3 {
-constexpr int NC = 2;                  // cells per thread along x: lane and lane + 32
-constexpr int TX = 32 * NC, BY = 8;    // owned tile 64 x 8
+constexpr int TX = 64, BY = 8;         // owned tile 64 x 8, two cells per thread: x = lane and lane + 32
 constexpr int NW = 10;                 // warps 0..7 own the tile rows, 8: +y halo row, 9: +x halo column
 constexpr int NT = 32 * NW;
 constexpr int BXW = TX + 8, BYH = BY + 2;  // TMA box 72 x 10: x in [i0-4, i0+68), y in [j0-1, j0+9)
@@ -37,17 +48,25 @@ constexpr int BOX = BXW * BYH;
 constexpr int NARR = 7;                // ex ey ez bx by bz sigma
 // ring stride of one box: rounded up to 128 bytes so every TMA destination is 128-byte aligned
 template <typename T> __host__ __device__ constexpr int boxs() { return (int)(((BOX * sizeof(T) + 127) / 128) * 128 / sizeof(T)); }
-constexpr int RING = 4;                // planes in flight
-constexpr int XR = BY + 2, XC = TX + 2;  // exchange planes of the new fields
+constexpr int RING = 4;                // stages in flight
 enum { AEX = 0, AEY, AEZ, ABX, ABY, ABZ, ASG };
-// byte offset of the RING mbarriers: after the ring, the three exchange planes and the two offset boxes
-template <typename T> __host__ __device__ constexpr size_t bars_offset() {
-    return (size_t)RING * NARR * boxs<T>() * sizeof(T) + 3 * 2 * XR * XC * sizeof(T) + 2 * BOX * sizeof(T);
-}
+// New planes in shared memory, two buffers each.  Those that neighbours read (Ez, Bx, By): nine dense rows
+// of 64 (the ninth is the +y halo row), then the +x halo column, then cells nobody reads for idle
+// lanes.  Those that are only stored (Ex, Ey, Bz): eight dense rows.
+constexpr int XCOL = 9 * TX, XBUF = 10 * TX, SBUF = BY * TX;
+enum { XEZ = 0, XBX, XBY };
+enum { SEX = 0, SEY, SBZ };
+template <typename T> __host__ __device__ constexpr int xoff(int a, int q) { return RING * NARR * boxs<T>() + (2 * a + q) * XBUF; }
+template <typename T> __host__ __device__ constexpr int soff(int a, int q) { return xoff<T>(3, 0) + (3 * q + a) * SBUF; }
+// byte offset of the RING mbarriers, the error flag and source planes, then the z tables
+template <typename T> __host__ __device__ constexpr size_t bars_offset() { return (size_t)soff<T>(0, 2) * sizeof(T); }
 template <typename T> __host__ __device__ constexpr size_t smem_bytes() { return bars_offset<T>() + RING * 8 + 16; }
 template <typename T> size_t smem_bytes_n(int N) {  // plus the z tables
-    return ((smem_bytes<T>() + 3 * (size_t)(N + 3) * sizeof(T)) + 15) / 16 * 16;
+    return smem_bytes<T>() + 3 * (size_t)(N + 3) * 2 * sizeof(T);
 }
+// the chunk offsets of Bz over the box, for the planes below k1 and for k1 itself, lie in the first
+// buffers of the stored planes: they are in registers before the third plane of the march writes there
+static_assert(2 * BOX <= 3 * SBUF, "the offset boxes fit the first store buffers");
 }  // namespace fs3
 
 // reciprocal used by the E update: one MUFU op in FP32 (about 1 ulp), exact division in FP64
@@ -74,322 +93,338 @@ __device__ __forceinline__ void recip3(double a, double b, double c, double &ra,
     rb = a * rab;
 }
 
-// per-thread state of the sweep (NC cells per thread); sweep_plane<PH>() advances
-// one z-plane with PH = (ktop - k) mod 4, so ring slots and exchange parities
-// are compile-time constants
+// per-thread state of the sweep; sweep_plane<PH>() advances one z-plane with PH = (ktop - k) mod 4, so ring
+// slots and buffer parities are compile-time constants
 template <typename T> struct SweepThread {
-    T *ring, *x_ez, *x_bxn, *x_byn;
+    T *sm;  // ring, then the new planes
     uint64_t *bars;
-    int *s_flag;
-    const CUtensorMap *maps;
-    unsigned plane_bytes;
-    int j, PS, N, k0, k1, klow, ktop, tid, i0, j0;
-    int role;  // 0: a row of the tile, 1: the +y halo row, 2: the +x halo column (warp-uniform; FP64)
-    int total;  // elements of each field array (bounds-checked builds)
-    int *err;
-    T rdy2, rdy, fy;  // per row: 1/(dy[j-1]+dy[j]), 1/dy[j], dtb/dy[j]
-    // per cell
-    int so[fs3::NC], xo[fs3::NC], i[fs3::NC], col[fs3::NC];
-    bool own[fs3::NC], vEx[fs3::NC], vEy[fs3::NC], vEz[fs3::NC];
-    T rdx2[fs3::NC], rdx[fs3::NC], fx[fs3::NC];
-    T oc0[fs3::NC], oci[fs3::NC], ocj[fs3::NC];  // Bz chunk offsets of the plane being updated: at, left of, below the cell
-    T ex1[fs3::NC], ey1[fs3::NC], exn[fs3::NC], eyn[fs3::NC], ezn[fs3::NC];
-    T bxo1[fs3::NC], byo1[fs3::NC], bxn[fs3::NC], byn[fs3::NC], acc[fs3::NC];
-    T sxk[fs3::NC], syk[fs3::NC], szk[fs3::NC], bxk[fs3::NC], byk[fs3::NC];  // sigma sums and own B of plane k
+    int *s_src;  // first and last plane with a source segment in the tile
+    const SweepMaps *maps;
+    int j, N, k0, k1, klow, ktop, i0, j0;
+    int role;     // 0: a row of the tile, 1: the +y halo row, 2: the +x halo column (warp-uniform)
+    int duty;     // 1: the thread issues the loads (a lane of the +y warp), 2: the stores (of the +x warp)
+    bool bad;     // a copy did not arrive
+    bool src;     // a source segment touches the tile in this step
+    int so, xo, xd, xr, i;         // first cell: in the box, in the new planes; its +y and the second one's +x neighbour; x index
+    // which components of the cells are updated: bits 0, 1 Ex and By, bits 2, 3 Ey and Bx (both: Ez too);
+    // edge: not all of them in some lane of the warp, which then keeps old values where they are not
+    unsigned upd;
+    bool edge;
+    Pair<T> rdy2, rdy, fy;         // per row: 1/(dy[j-1]+dy[j]), 1/dy[j], dtb/dy[j]
+    Pair<T> lam, c4;               // FP32: 2 lambda / (dt/4), c4 / (dt/4); FP64: 2 lambda, c4
+    Pair<T> rdx2, rdx, fx;
+    Pair<T> oc0, oci, ocj;  // Bz chunk offsets of the plane being updated: at, left of, below the cells
+    Pair<T> ex1, ey1, exn, eyn, ezn;
+    Pair<T> bxo1, byo1, bxn, byn, acc;
+    Pair<T> sxk, syk, szk, bxk, byk, bxj, byi;  // of plane k: sigma sums, own B, Bx below and By left of the cell
 };
 
-template <typename T, int PH, int ROLE>
-__device__ __forceinline__ bool sweep_plane(SweepThread<T> &t, int k, unsigned rp, const StepScalars<T> &s,
-                                            const T *__restrict__ zt, const FieldSet<T> &out,
-                                            const SourceTable<T> &src, bool src_tile) {
+// the old value of the cells whose bit of m (bits 0, 1) is not set
+template <typename T> __device__ __forceinline__ void keep(Pair<T> &v, Pair<T> old, unsigned m) {
+    if (!(m & 1u)) v.a = old.a;
+    if (!(m & 2u)) v.b = old.b;
+}
+// the thread's two cells at offset o
+template <typename T> __device__ __forceinline__ Pair<T> cells(const T *p, int o) { return pair<T>(p[o], p[o + 32]); }
+template <typename T> __device__ __forceinline__ void put_cells(T *p, int o, Pair<T> v) { p[o] = v.a; p[o + 32] = v.b; }
+
+// sigma sums and B of the plane in the B and sigma boxes p
+template <typename T> __device__ __forceinline__ void carry_plane(SweepThread<T> &t, const T *p) {
     using namespace fs3;
     constexpr int BS = boxs<T>();
-    constexpr int S0 = PH, S1 = (PH + 1) & 3;
+    const T *sg = p + ASG * BS;
+    const int so = t.so;
+    const Pair<T> a = cells(sg, so), b = cells(sg, so - 1), c = cells(sg, so - BXW), d = cells(sg, so - BXW - 1);
+    t.sxk = a + c;
+    t.syk = a + b;
+    t.szk = t.sxk + b + d;
+    t.bxk = cells(p + ABX * BS, so);
+    t.byk = cells(p + ABY * BS, so);
+    t.bxj = cells(p + ABX * BS, so - BXW);
+    t.byi = cells(p + ABY * BS, so - 1);
+}
+// the loading thread: stage k into slot q
+template <typename T> __device__ __forceinline__ void load_stage(const SweepThread<T> &t, int k, int q) {
+    using namespace fs3;
+    uint64_t *b = t.bars + q;
+    T *dst = t.sm + q * NARR * boxs<T>();
+    auto box = [&](int a, int z) { tma_load_3d(dst + a * boxs<T>(), t.maps->m + a, t.i0, t.j0, z + 1, b); };
+    mbar_expect_tx(b, (unsigned)(NARR * BOX * sizeof(T)));
+    box(AEX, k);
+    box(AEY, k);
+    box(AEZ, k);
+    box(ABZ, k);
+    box(ASG, k - 1);
+    // the air plane is the boundary's output: a top chunk launched early (programmatic dependent launch after
+    // the boundary's last stage) waits for it here and not before (no-op without the launch attribute)
+    if (k == 0) pdl_wait_prev();
+    box(ABX, k - 1);
+    box(ABY, k - 1);
+}
+
+// Planes of a march: the first one (k = ktop: E of the halo plane, or the zero bottom; nothing stored), the
+// second (no B below it in the chunk), the inner ones, and k0 - 1 (only B(k0)).  Compiled apart: the inner
+// planes' code has no condition on k but the two at the end of the ring.
+enum { FIRST, SECOND, INNER, LAST };
+
+template <typename T, int PH, int KIND, int ROLE>
+__device__ __forceinline__ void sweep_plane(SweepThread<T> &t, int k, unsigned rp, const StepScalars<T> &s,
+                                            const Pair<T> *zt, const SourceTable<T> &src) {
+    using namespace fs3;
+    typedef Pair<T> P;
+    constexpr int BS = boxs<T>();
     constexpr int QE = PH & 1, QB = (PH + 1) & 1;
-    constexpr int XP2 = XR * XC;
-    const int zi = k - t.klow;  // z tables: rdz, rdzs, dzk of plane klow + zi
+    constexpr bool doB = KIND == INNER || KIND == LAST, doE = KIND != LAST;
+    zt += 3 * (k - t.klow);  // dtb/dz, 1/(dz[k-1]+dz[k]), dz of plane k
     // Roles (one compiled copy each, FP64 only): the row warps update and store every component; the
     // +y halo row warp only produces what the tile's last row reads from it (Ex and Ez for By there,
     // By for Bz), the +x halo column warp what the tile's last column reads (Ey and Ez for Bx there,
     // Bx for Bz).  Every copy passes the one barrier per plane in the same order.
-    constexpr bool rX = ROLE != 2, rY = ROLE != 1, rR = ROLE == 0;
+    constexpr bool rX = ROLE != 2, rY = ROLE != 1;
+    const bool rows = sizeof(T) == 8 ? ROLE == 0 : t.role == 0;
+    T *const sm = t.sm;
     // ---- B_new(k+1) from E_new(k+1) (own + neighbours) and E_new(k+2)
-    const bool doB = k + 1 < t.k1;
-    if (doB) {
-        const T fz = zt[3 * (zi + 1)] * s.dtb;  // dtb / dz(k+1)
-#pragma unroll
-        for (int c = 0; c < NC; c++) {
-            if constexpr (rY) {
-                const T ezj = t.x_ez[QB * XP2 + t.xo[c] + XC];
-                const T bx = t.bxo1[c] + (t.ey1[c] - t.eyn[c]) * fz - (ezj - t.ezn[c]) * t.fy;
-                t.bxn[c] = t.vEy[c] ? bx : t.bxo1[c];
-            }
-            if constexpr (rX) {
-                const T ezi = t.x_ez[QB * XP2 + t.xo[c] + 1];
-                const T by = t.byo1[c] + (ezi - t.ezn[c]) * t.fx[c] - (t.ex1[c] - t.exn[c]) * fz;
-                t.byn[c] = t.vEx[c] ? by : t.byo1[c];
-            }
-            if (rR && t.own[c] && TCSEM_IN(t.col[c] + (k + 2) * t.PS, t.total, t.err)) {
-                const int o = t.col[c] + (k + 2) * t.PS;
-                out.bx[o] = t.bxn[c];
-                out.by[o] = t.byn[c];
-            }
+    if constexpr (doB) {
+        const P fz = zt[3];
+        const T *ez = sm + xoff<T>(XEZ, QB);
+        if constexpr (rY) {
+            const P ezj = cells(ez, t.xd);
+            t.bxn = fma(t.ezn - ezj, t.fy, fma(t.ey1 - t.eyn, fz, t.bxo1));
+        }
+        if constexpr (rX) {
+            const P ezi = pair<T>(ez[t.xo + 1], ez[t.xr]);
+            t.byn = fma(t.exn - t.ex1, fz, fma(ezi - t.ezn, t.fx, t.byo1));
+        }
+        if (t.edge) {
+            keep(t.bxn, t.bxo1, t.upd >> 2);
+            keep(t.byn, t.byo1, t.upd);
         }
     }
     // ---- E_new(k)
-#pragma unroll
-    for (int c = 0; c < NC; c++) {
-        t.ex1[c] = t.exn[c];
-        t.ey1[c] = t.eyn[c];
-    }
-    if (k >= t.k0) {
-        const bool upd = k < t.N, lo = k < t.k1;
-        const T rzs = zt[3 * zi + 1];
-#pragma unroll
-        for (int c = 0; c < NC; c++) {
-            const T *p0 = t.ring + S0 * NARR * BS + t.so[c], *p1 = t.ring + S1 * NARR * BS + t.so[c];
-            const T a1 = p1[ASG * BS], b1 = p1[ASG * BS - 1], c1 = p1[ASG * BS - BXW], d1 = p1[ASG * BS - BXW - 1];
-            const T bym = p1[ABY * BS], bxm = p1[ABX * BS];
-            const T sx1 = a1 + c1, sy1 = a1 + b1, sz1 = sx1 + b1 + d1;
-            const T ezo = p0[AEZ * BS];
-            T exo = T(0), eyo = T(0);
-            if constexpr (rX) exo = p0[AEX * BS];
-            if constexpr (rY) eyo = p0[AEY * BS];
-            if (upd) {
-                const T bz = p0[ABZ * BS] + t.oc0[c];
-                const T byi = p0[ABY * BS - 1], bxj = p0[ABX * BS - BXW];
-                // DuFort-Frankel update (ElectricalFiled.cu:89-345) of the three components, computed for
-                // every cell and kept where the component is updated; s.dt carries the 1/4 of the sigma sums
-                const T sdx = (t.sxk[c] + sx1) * s.dt, sdy = (t.syk[c] + sy1) * s.dt, sdz = t.szk[c] * s.dt;
-                const T cz = (t.byk[c] - byi) * t.rdx2[c] - (t.bxk[c] - bxj) * t.rdy2;
-                if constexpr (sizeof(T) == 8) {
-                    // FP64, bound by the FP64 pipe: with D = lam2 + sigma dt, the update
-                    // (lam2 - sigma dt)/D E + c4/D curl is written (2 lam2 E + c4 curl)/D - E -- three
-                    // operations per component after 1/D instead of five.  (In FP32, where 1/D is an
-                    // approximate reciprocal, the same form raised the trace error of a long whole run on
-                    // 142 x 36 x 25 cells to 1.02 % of its peak, and saved 0.3 % of the step time.)
-                    T rx, ry, rz;
-                    recip3(s.lam2 + sdx, s.lam2 + sdy, s.lam2 + sdz, rx, ry, rz);
-                    const T l2 = s.lam2 + s.lam2;
-                    if constexpr (rX) {
-                        const T bzj = p0[ABZ * BS - BXW] + t.ocj[c];
-                        const T cx = (bz - bzj) * t.rdy2 - (t.byk[c] - bym) * rzs;
-                        const T ex = fma(fma(s.c4, cx, l2 * exo), rx, -exo);
-                        t.exn[c] = t.vEx[c] ? ex : exo;
-                    }
-                    if constexpr (rY) {
-                        const T bzi = p0[ABZ * BS - 1] + t.oci[c];
-                        const T cy = (t.bxk[c] - bxm) * rzs - (bz - bzi) * t.rdx2[c];
-                        const T ey = fma(fma(s.c4, cy, l2 * eyo), ry, -eyo);
-                        t.eyn[c] = t.vEy[c] ? ey : eyo;
-                    }
-                    const T ez = fma(fma(s.c4, cz, l2 * ezo), rz, -ezo);
-                    t.ezn[c] = t.vEz[c] ? ez : ezo;
-                } else {
-                    if constexpr (rX) {
-                        const T bzj = p0[ABZ * BS - BXW] + t.ocj[c];
-                        const T cx = (bz - bzj) * t.rdy2 - (t.byk[c] - bym) * rzs;
-                        const T rx = rcp_fast(s.lam2 + sdx);
-                        const T ex = ((s.lam2 - sdx) * rx) * exo + (s.c4 * rx) * cx;
-                        t.exn[c] = t.vEx[c] ? ex : exo;
-                    }
-                    if constexpr (rY) {
-                        const T bzi = p0[ABZ * BS - 1] + t.oci[c];
-                        const T cy = (t.bxk[c] - bxm) * rzs - (bz - bzi) * t.rdx2[c];
-                        const T ry = rcp_fast(s.lam2 + sdy);
-                        const T ey = ((s.lam2 - sdy) * ry) * eyo + (s.c4 * ry) * cy;
-                        t.eyn[c] = t.vEy[c] ? ey : eyo;
-                    }
-                    const T rz = rcp_fast(s.lam2 + sdz);
-                    const T ez = ((s.lam2 - sdz) * rz) * ezo + (s.c4 * rz) * cz;
-                    t.ezn[c] = t.vEz[c] ? ez : ezo;
-                }
+    if constexpr (doE) {
+        t.ex1 = t.exn;
+        t.ey1 = t.eyn;
+        const T *p0 = sm + PH * NARR * BS;
+        const int so = t.so;
+        const P sx0 = t.sxk, sy0 = t.syk, sz0 = t.szk, bx0 = t.bxk, by0 = t.byk, bxj = t.bxj, byi = t.byi;
+        carry_plane(t, p0);  // plane k-1, the next one up
+        const P ezo = cells(p0 + AEZ * BS, so);
+        P exo = dup<T>(T(0)), eyo = exo;
+        if constexpr (rX) exo = cells(p0 + AEX * BS, so);
+        if constexpr (rY) eyo = cells(p0 + AEY * BS, so);
+        if (KIND != FIRST || k < t.N) {
+            const P bz = cells(p0 + ABZ * BS, so) + t.oc0;
+            // DuFort-Frankel update (ElectricalFiled.cu:89-345) of the three components, computed for
+            // every cell and kept where the component is updated; s.dt carries the 1/4 of the sigma sums
+            const P sx = sx0 + t.sxk, sy = sy0 + t.syk, lam = t.lam, c4 = t.c4, rdy2 = t.rdy2, rz2 = zt[1];
+            const P cz = fma(by0 - byi, t.rdx2, -((bx0 - bxj) * rdy2));
+            P cx, cy;
+            if constexpr (rX) cx = fma(bz - (cells(p0 + ABZ * BS, so - BXW) + t.ocj), rdy2, -((by0 - t.byk) * rz2));
+            if constexpr (rY) cy = fma(bx0 - t.bxk, rz2, -((bz - (cells(p0 + ABZ * BS, so - 1) + t.oci)) * t.rdx2));
+            if constexpr (sizeof(T) == 8) {
+                const P dt = dup<T>(s.dt), Dx = fma(sx, dt, lam), Dy = fma(sy, dt, lam), Dz = fma(sz0, dt, lam);
+                // FP64, bound by the FP64 pipe: with D = lam2 + sigma dt, the update
+                // (lam2 - sigma dt)/D E + c4/D curl is written (2 lam2 E + c4 curl)/D - E -- three
+                // operations per component after 1/D instead of five.  (In FP32, where 1/D is an
+                // approximate reciprocal, the same form raised the trace error of a long whole run on
+                // 142 x 36 x 25 cells to 1.02 % of its peak, and saved 0.3 % of the step time.)
+                P rx, ry, rz;
+                recip3(Dx.a, Dy.a, Dz.a, rx.a, ry.a, rz.a);
+                recip3(Dx.b, Dy.b, Dz.b, rx.b, ry.b, rz.b);
+                const P l2 = lam + lam;
+                if constexpr (rX) t.exn = fma(fma(c4, cx, l2 * exo), rx, -exo);
+                if constexpr (rY) t.eyn = fma(fma(c4, cy, l2 * eyo), ry, -eyo);
+                t.ezn = fma(fma(c4, cz, l2 * ezo), rz, -ezo);
             } else {
-                t.exn[c] = exo;
-                t.eyn[c] = eyo;
-                t.ezn[c] = ezo;
+                auto rcp = [](P d) { return pair<T>(rcp_fast(d.a), rcp_fast(d.b)); };
+                // numerator and denominator divided by dt/4: no product with dt per cell
+                const P rx = rcp(lam + sx), ry = rcp(lam + sy), rz = rcp(lam + sz0);
+                t.exn = fma((lam - sx) * rx, exo, (c4 * rx) * cx);
+                t.eyn = fma((lam - sy) * ry, eyo, (c4 * ry) * cy);
+                t.ezn = fma((lam - sz0) * rz, ezo, (c4 * rz) * cz);
             }
-            t.bxo1[c] = t.bxk[c];  // B_old(k) for the next plane's B update
-            t.byo1[c] = t.byk[c];
-            t.bxk[c] = bxm;
-            t.byk[c] = bym;
-            t.sxk[c] = sx1;
-            t.syk[c] = sy1;
-            t.szk[c] = sz1;
-        }
-        // AddTx_*: subtracted after the update of the cell, on the planes where a segment meets the tile
-        if (upd && src_tile && s.wave != T(0) && k >= t.s_flag[1] && k <= t.s_flag[2]) {
+            if (t.edge) {
+                if constexpr (rX) keep(t.exn, exo, t.upd);
+                if constexpr (rY) keep(t.eyn, eyo, t.upd >> 2);
+                keep(t.ezn, ezo, t.upd & (t.upd >> 2));
+            }
+            // AddTx_*: subtracted after the update of the cell, on the planes where a segment meets the tile
+            if (t.src && k >= t.s_src[0] && k <= t.s_src[1]) {
+                T e[3][2] = {{t.exn.a, t.exn.b}, {t.eyn.a, t.eyn.b}, {t.ezn.a, t.ezn.b}};
 #pragma unroll
-            for (int c = 0; c < NC; c++) {
-                if (!(t.vEx[c] || t.vEy[c])) continue;
-                for (int q = 0; q < src.nseg; q++) {
-                    const int cp = src.comp[q];
-                    int d;
-                    if (cp == 0) { if (t.j != src.j[q] || k != src.k[q]) continue; d = t.i[c] - src.i[q]; }
-                    else if (cp == 1) { if (t.i[c] != src.i[q] || k != src.k[q]) continue; d = t.j - src.j[q]; }
-                    else { if (t.i[c] != src.i[q] || t.j != src.j[q]) continue; d = k - src.k[q]; }
-                    if (d < 0 || d >= src.count[q]) continue;
-                    const T v = s.wave * src.coef[src.off[q] + d];
-                    if (cp == 0) t.exn[c] -= v; else if (cp == 1) t.eyn[c] -= v; else t.ezn[c] -= v;
+                for (int c = 0; c < 2; c++) {
+                    if (!(t.upd & (5u << c))) continue;
+                    const int i = t.i + 32 * c;
+                    for (int q = 0; q < src.nseg; q++) {
+                        const int cp = src.comp[q];
+                        int d;
+                        if (cp == 0) { if (t.j != src.j[q] || k != src.k[q]) continue; d = i - src.i[q]; }
+                        else if (cp == 1) { if (i != src.i[q] || k != src.k[q]) continue; d = t.j - src.j[q]; }
+                        else { if (i != src.i[q] || t.j != src.j[q]) continue; d = k - src.k[q]; }
+                        if (d < 0 || d >= src.count[q]) continue;
+                        const T v = s.wave * src.coef[src.off[q] + d];
+                        if (cp == 0) e[0][c] -= v; else if (cp == 1) e[1][c] -= v; else e[2][c] -= v;
+                    }
                 }
+                t.exn = pair<T>(e[0][0], e[0][1]);
+                t.eyn = pair<T>(e[1][0], e[1][1]);
+                t.ezn = pair<T>(e[2][0], e[2][1]);
             }
+        } else {
+            t.exn = exo;
+            t.eyn = eyo;
+            t.ezn = ezo;
         }
-#pragma unroll
-        for (int c = 0; c < NC; c++) {
-            if (rR && upd && lo && t.own[c] && TCSEM_IN(t.col[c] + (k + 1) * t.PS, t.total, t.err)) {
-                const int o = t.col[c] + (k + 1) * t.PS;
-                out.ex[o] = t.exn[c];
-                out.ey[o] = t.eyn[c];
-                out.ez[o] = t.ezn[c];
-            }
-            t.x_ez[QE * XP2 + t.xo[c]] = t.ezn[c];  // publish Ez_new(k)
+        t.bxo1 = bx0;  // B_old(k) for the next plane's B update
+        t.byo1 = by0;
+        put_cells(sm + xoff<T>(XEZ, QE), t.xo, t.ezn);  // publish Ez_new(k)
+        if (KIND != FIRST && rows) {
+            put_cells(sm + soff<T>(SEX, QE), t.xo, t.exn);
+            put_cells(sm + soff<T>(SEY, QE), t.xo, t.eyn);
         }
     }
-    if (doB) {  // publish B_new(k+1): Bx where Bz reads it (rows, +x column), By likewise (rows, +y row)
-#pragma unroll
-        for (int c = 0; c < NC; c++) {
-            if constexpr (rY) t.x_bxn[QB * XP2 + t.xo[c]] = t.bxn[c];
-            if constexpr (rX) t.x_byn[QB * XP2 + t.xo[c]] = t.byn[c];
-        }
+    if constexpr (doB) {  // publish B_new(k+1): Bx where Bz reads it (rows, +x column), By likewise (rows, +y row)
+        if constexpr (rY) put_cells(sm + xoff<T>(XBX, QB), t.xo, t.bxn);
+        if constexpr (rX) put_cells(sm + xoff<T>(XBY, QB), t.xo, t.byn);
     }
-    // plane k-2 is read by the next plane
-    if (k - 2 >= t.klow && !mbar_wait_bounded(t.bars + ((PH + 2) & 3), rp ^ (unsigned)((PH + 2) >> 2))) *t.s_flag = 1;
+    // stage k-1 is read by the next plane; a thread whose wait gave up does not wait again.  Slot 3 is one
+    // phase ahead: it carried plane ktop's B and sigma first.
+    constexpr int NS = (PH + 1) & 3;
+    if (doE && k > t.k0 && !t.bad) t.bad = !mbar_wait_bounded(t.bars + NS, rp ^ (unsigned)((PH + 1) >> 2) ^ (NS == 3 ? 1u : 0u));
+    async_shared_fence();  // the new planes are read by the TMA
+    if (t.duty == 2) bulk_wait_read();  // ... which is done with the buffers the next plane writes
     __syncthreads();
-    if (*t.s_flag) {  // a copy did not arrive: let the copies still in flight (planes k-2, k-3) land first
-        if (t.tid == 0) {
-            if (k - 2 >= t.klow) mbar_wait_bounded(t.bars + ((PH + 2) & 3), rp ^ (unsigned)((PH + 2) >> 2));
-            if (k - 3 >= t.klow) mbar_wait_bounded(t.bars + ((PH + 3) & 3), rp ^ (unsigned)((PH + 3) >> 2));
+    if (t.duty) {
+        if (t.duty == 2) {  // store E(k), B(k+1) and, summed after the barrier of plane k+1, Bz(k+2)
+            if constexpr (KIND == SECOND || KIND == INNER) {
+                tma_store_3d(t.maps->o + 0, sm + soff<T>(SEX, QE), t.i0, t.j0, k);
+                tma_store_3d(t.maps->o + 1, sm + soff<T>(SEY, QE), t.i0, t.j0, k);
+                tma_store_3d(t.maps->o + 2, sm + xoff<T>(XEZ, QE), t.i0, t.j0, k);
+            }
+            if constexpr (doB) {
+                tma_store_3d(t.maps->o + 3, sm + xoff<T>(XBX, QB), t.i0, t.j0, k + 1);
+                tma_store_3d(t.maps->o + 4, sm + xoff<T>(XBY, QB), t.i0, t.j0, k + 1);
+                if (k + 2 < t.k1) tma_store_3d(t.maps->o + 5, sm + soff<T>(SBZ, QB), t.i0, t.j0, k + 2);
+            }
+            bulk_commit();
+        } else if (doE && k - RING >= t.k0) {  // the slot takes stage k-4
+            load_stage(t, k - RING, PH);
         }
-        return false;
-    }
-    // plane k is no longer read: its ring slot takes plane k-4
-    if (t.tid == 0 && k - RING >= t.klow && k >= t.k0) {
-        if (k - RING < 0) pdl_wait_prev();  // the air plane is the boundary's output (no-op without the launch attribute)
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        uint64_t *b = t.bars + S0;
-        mbar_expect_tx(b, t.plane_bytes);
-#pragma unroll
-        for (int a = 0; a < NARR; a++) tma_load_3d(t.ring + (S0 * NARR + a) * BS, t.maps + a, t.i0, t.j0, k - RING + 1, b);
     }
     // ---- Bz(k+1) = Bz(k+2) + dz (dBx/dx + dBy/dy), for the tile's own rows
-    if (doB && rR) {
-        const T dz = zt[3 * (zi + 1) + 2];
-#pragma unroll
-        for (int c = 0; c < NC; c++) {
-            t.acc[c] += dz * ((t.x_bxn[QB * XP2 + t.xo[c] + 1] - t.bxn[c]) * t.rdx[c] +
-                              (t.x_byn[QB * XP2 + t.xo[c] + XC] - t.byn[c]) * t.rdy);
-            if (t.own[c] && TCSEM_IN(t.col[c] + (k + 2) * t.PS, t.total, t.err)) out.bz[t.col[c] + (k + 2) * t.PS] = t.acc[c];
-        }
+    if (doB && rows) {
+        const T *bx = sm + xoff<T>(XBX, QB), *by = sm + xoff<T>(XBY, QB);
+        const P bxr = pair<T>(bx[t.xo + 1], bx[t.xr]), byu = cells(by, t.xd);
+        t.acc = fma(zt[5], fma(bxr - t.bxn, t.rdx, (byu - t.byn) * t.rdy), t.acc);
+        put_cells(sm + soff<T>(SBZ, QE), t.xo, t.acc);
     }
-    return true;
+}
+
+// the cells' Bz chunk offsets from one of the two offset boxes
+template <typename T> __device__ __forceinline__ void set_offsets(SweepThread<T> &t, const T *box) {
+    t.oc0 = cells(box, t.so);
+    t.oci = cells(box, t.so - 1);
+    t.ocj = cells(box, t.so - fs3::BXW);
 }
 
 // the z-march of one warp through the chunk, in the copy of the plane code for its role
 template <typename T, int ROLE>
-__device__ __forceinline__ bool sweep_march(SweepThread<T> &t, const StepScalars<T> &s, const T *__restrict__ s_z,
-                                            const FieldSet<T> &out, const SourceTable<T> &src, bool src_tile,
-                                            const T *s_oc);
-
-// the cells' Bz chunk offsets from one of the two offset boxes
-template <typename T> __device__ __forceinline__ void set_offsets(SweepThread<T> &t, const T *box) {
-#pragma unroll
-    for (int q = 0; q < fs3::NC; q++) {
-        t.oc0[q] = box[t.so[q]];
-        t.oci[q] = box[t.so[q] - 1];
-        t.ocj[q] = box[t.so[q] - fs3::BXW];
-    }
-}
-
-template <typename T, int ROLE>
-__device__ __forceinline__ bool sweep_march(SweepThread<T> &t, const StepScalars<T> &s, const T *__restrict__ s_z,
-                                            const FieldSet<T> &out, const SourceTable<T> &src, bool src_tile,
-                                            const T *s_oc) {
+__device__ __forceinline__ void sweep_march(SweepThread<T> &t, const StepScalars<T> &s, const Pair<T> *s_z,
+                                            const SourceTable<T> &src, const T *s_oc) {
     using namespace fs3;
-    bool ok = true;
-    unsigned rp = 0;  // parity of the ring round
-    const int ktop = t.ktop;
-    for (int k = ktop; ok && k >= t.k0 - 1; k -= RING, rp ^= 1u) {
-        ok = sweep_plane<T, 0, ROLE>(t, k, rp, s, s_z, out, src, src_tile);
-        if (k == ktop) set_offsets(t, s_oc);
-        if (!ok || k - 1 < t.k0 - 1) break;
-        ok = sweep_plane<T, 1, ROLE>(t, k - 1, rp, s, s_z, out, src, src_tile);
-        if (!ok || k - 2 < t.k0 - 1) break;
-        ok = sweep_plane<T, 2, ROLE>(t, k - 2, rp, s, s_z, out, src, src_tile);
-        if (!ok || k - 3 < t.k0 - 1) break;
-        ok = sweep_plane<T, 3, ROLE>(t, k - 3, rp, s, s_z, out, src, src_tile);
+    const int k0 = t.k0;
+    sweep_plane<T, 0, FIRST, ROLE>(t, t.ktop, 0u, s, s_z, src);
+    set_offsets(t, s_oc);
+    // the inner planes k = ktop - 2 .. k0 begin in phase 2; rp: parity of the ring round
+    int k = t.ktop - 1;
+    sweep_plane<T, 1, SECOND, ROLE>(t, k, 0u, s, s_z, src);
+    unsigned rp = 0;
+    int left = 2;  // phase of the plane after the last inner one
+    while (--k >= k0) {
+        sweep_plane<T, 2, INNER, ROLE>(t, k, rp, s, s_z, src);
+        if (--k < k0) { left = 3; break; }
+        sweep_plane<T, 3, INNER, ROLE>(t, k, rp, s, s_z, src);
+        rp ^= 1u;
+        if (--k < k0) { left = 0; break; }
+        sweep_plane<T, 0, INNER, ROLE>(t, k, rp, s, s_z, src);
+        if (--k < k0) { left = 1; break; }
+        sweep_plane<T, 1, INNER, ROLE>(t, k, rp, s, s_z, src);
     }
-    return ok;
+    if (left == 0) sweep_plane<T, 0, LAST, ROLE>(t, k, rp, s, s_z, src);
+    else if (left == 1) sweep_plane<T, 1, LAST, ROLE>(t, k, rp, s, s_z, src);
+    else if (left == 2) sweep_plane<T, 2, LAST, ROLE>(t, k, rp, s, s_z, src);
+    else sweep_plane<T, 3, LAST, ROLE>(t, k, rp, s, s_z, src);
 }
 
 // one CTA of the sweep: tile (bx, by) of z-chunk c with the step scalars s.  FRESH: the chunk
 // totals tin may have been written by another CTA of the same launch (persistent schedule).
 template <typename T, bool FRESH = false>
-__device__ __forceinline__ void sweep_cta(const SweepMaps &maps, const Geom &g, const FieldSet<T> &out,
-                                          const T *__restrict__ tin, T *__restrict__ tout, const Axis<T> &ax,
-                                          StepScalars<T> s, const SourceTable<T> &src, const ZChunks &zc, int bx,
-                                          int by, int c, int *err) {
+__device__ __forceinline__ void sweep_cta(const SweepMaps &maps, const Geom &g, const T *__restrict__ tin,
+                                          T *__restrict__ tout, const Axis<T> &ax, StepScalars<T> s,
+                                          const SourceTable<T> &src, const ZChunks &zc, int bx, int by, int c, int *err) {
     using namespace fs3;
     constexpr int BS = boxs<T>();
     extern __shared__ __align__(128) unsigned char smem_raw[];
     SweepThread<T> t;
-    t.ring = reinterpret_cast<T *>(smem_raw);
-    t.x_ez = t.ring + RING * NARR * BS;  // [2][XR][XC]
-    t.x_bxn = t.x_ez + 2 * XR * XC;
-    t.x_byn = t.x_bxn + 2 * XR * XC;
-    T *s_oc = t.x_byn + 2 * XR * XC;  // [BYH][BXW] chunk offsets of Bz for planes < k1
-    T *s_oc1 = s_oc + BOX;            // ... for plane k1
-    t.bars = reinterpret_cast<uint64_t *>(s_oc1 + BOX);  // 8-byte aligned: every region above has an even size
-    static_assert(bars_offset<T>() % 8 == 0, "mbarriers need 8-byte alignment");
-    t.s_flag = reinterpret_cast<int *>(t.bars + RING);
-    T *s_z = reinterpret_cast<T *>(reinterpret_cast<unsigned char *>(t.bars) + RING * 8 + 16);  // [N+3][3]
-    t.maps = maps.m;
+    t.sm = reinterpret_cast<T *>(smem_raw);
+    T *s_oc = t.sm + soff<T>(0, 0);  // [BYH][BXW] chunk offsets of Bz for planes < k1
+    T *s_oc1 = s_oc + BOX;           // ... for plane k1
+    t.bars = reinterpret_cast<uint64_t *>(smem_raw + bars_offset<T>());
+    static_assert(bars_offset<T>() % 128 == 0, "the new planes are whole 128-byte lines");
+    t.s_src = reinterpret_cast<int *>(t.bars + RING);
+    Pair<T> *s_z = reinterpret_cast<Pair<T> *>(smem_raw + smem_bytes<T>());  // [N+3][3], each value twice
+    t.maps = &maps;
 
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    t.tid = tid;
     t.i0 = bx * TX;
     t.j0 = by * BY;
-    const int L = g.L, M = g.M, N = g.N, XP = g.XP;
+    const int L = g.L, M = g.M, N = g.N, XP = g.XP, PS = (int)g.PS;
     t.N = N;
-    t.PS = (int)g.PS;
-    t.total = (int)g.total();
-    t.err = err;
     t.k0 = zc.plane(c);
     t.k1 = zc.plane(c + 1);
-    const int ty = w < 9 ? w : lane;
+    // rows: cells x = lane, lane + 32 of row w; column warp: one cell per lane, x = 64 of row `lane`
+    const bool column = w == 9;
+    const int ty = column ? lane : w;
     t.role = w < 8 ? 0 : (w == 8 ? 1 : 2);
+    t.duty = lane == 0 ? t.role : 0;
     t.j = t.j0 + ty;
-    const bool rowok = w < 9 || lane <= BY;
-    t.rdy2 = (rowok && t.j >= 1 && t.j < M) ? ax.rdy2[t.j] : T(0);
-    t.rdy = (rowok && t.j < M) ? ax.rdy[t.j] : T(0);
-    t.fy = t.rdy * s.dtb;
-#pragma unroll
-    for (int q = 0; q < NC; q++) {
-        const int tx = w < 9 ? lane + 32 * q : TX;
-        const bool act = w < 9 || (q == 0 && lane <= BY);
-        const int i = t.i0 + tx;
-        t.i[q] = i;
-        t.own[q] = act && ty < BY && tx < TX && i < L && t.j < M;
-        t.col[q] = (t.j + 1) * XP + (i + 4);
-        t.so[q] = act ? (ty + 1) * BXW + (tx + 4) : BXW + 4;
-        t.xo[q] = act ? ty * XC + tx : XR * XC - 1;  // inactive slots publish into a cell nobody reads
-        t.vEx[q] = act && t.j >= 1 && t.j < M && i < L;
-        t.vEy[q] = act && i >= 1 && i < L && t.j < M;
-        t.vEz[q] = t.vEx[q] && i >= 1;
-        t.rdx2[q] = t.vEy[q] ? ax.rdx2[i] : T(0);
-        t.rdx[q] = (act && i < L) ? ax.rdx[i] : T(0);
-        t.fx[q] = t.rdx[q] * s.dtb;
-    }
-    t.ktop = t.k1 < N ? t.k1 : N;  // first plane: the chunk's halo plane below, or the zero bottom
-    t.klow = t.k0 - 1 >= -1 ? t.k0 - 1 : -1;
-    t.plane_bytes = (unsigned)(NARR * BOX * sizeof(T));
-    const int ktop = t.ktop, klow = t.klow;
+    t.i = t.i0 + (column ? TX : lane);
+    const bool rowok = !column || lane <= BY;
+    t.so = rowok ? (ty + 1) * BXW + (column ? TX : lane) + 4 : BXW + 4;
+    t.xo = column ? XCOL + lane : ty * TX + lane;  // the column's idle lanes and second cells: cells nobody reads
+    t.xd = t.xo + (column ? 1 : TX);
+    t.xr = column ? t.xo : lane < 31 ? t.xo + 33 : XCOL + ty;
+    const T rdy = (rowok && t.j < M) ? ax.rdy[t.j] : T(0);
+    t.rdy2 = (dup<T>((rowok && t.j >= 1 && t.j < M) ? ax.rdy2[t.j] : T(0)));
+    t.rdy = (dup<T>(rdy));
+    t.fy = (dup<T>(rdy * s.dtb));
     s.dt *= T(0.25);  // the sweep forms sigma sums of four cells: 0.25 * sum * dt
+    t.lam = (dup<T>(sizeof(T) == 4 ? s.lam2 / s.dt : s.lam2));
+    t.c4 = (dup<T>(sizeof(T) == 4 ? s.c4 / s.dt : s.c4));
+    T r2[2], r1[2];
+    t.upd = 0;
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+        const bool act = rowok && (q == 0 || !column);
+        const int i = t.i + 32 * q;
+        const bool ux = act && t.j >= 1 && t.j < M && i < L, uy = act && i >= 1 && i < L && t.j < M;
+        t.upd |= (ux ? 1u << q : 0u) | (uy ? 4u << q : 0u);
+        r2[q] = uy ? ax.rdx2[i] : T(0);
+        r1[q] = (act && i < L) ? ax.rdx[i] : T(0);
+    }
+    t.edge = __any_sync(0xffffffffu, t.upd != 15u);
+    t.rdx2 = pair<T>(r2[0], r2[1]);
+    t.rdx = pair<T>(r1[0], r1[1]);
+    t.fx = pair<T>(r1[0] * s.dtb, r1[1] * s.dtb);
+    t.ktop = t.k1 < N ? t.k1 : N;  // first plane: the chunk's halo plane below, or the zero bottom
+    t.klow = t.k0 - 1;
+    const int ktop = t.ktop, klow = t.klow;
     for (int e = tid; e <= ktop + 1 - klow; e += NT) {
         const int k = klow + e;
         const bool in = k >= 0 && k < N;
-        s_z[3 * e] = in ? ax.rdz[k] : T(0);
-        s_z[3 * e + 1] = in ? ax.rdzs[k] : T(0);
-        s_z[3 * e + 2] = in ? ax.dzk[k] : T(0);
+        s_z[3 * e] = dup<T>(in ? ax.rdz[k] * s.dtb : T(0));
+        s_z[3 * e + 1] = dup<T>(in ? ax.rdzs[k] : T(0));
+        s_z[3 * e + 2] = dup<T>(in ? ax.dzk[k] : T(0));
     }
 
     bool src_tile = false;  // tile-uniform: does any source segment touch this tile, and on which planes?
@@ -405,23 +440,21 @@ __device__ __forceinline__ void sweep_cta(const SweepMaps &maps, const Geom &g, 
             sk1 = max(sk1, c1);
         }
     }
+    t.src = src_tile && s.wave != T(0);
     if (tid == 0) {
         for (int r = 0; r < RING; r++) mbar_init(t.bars + r, 1);
         mbar_init_fence();
-        t.s_flag[0] = 0;
-        t.s_flag[1] = sk0;  // read by the source epilogue, after the barrier below
-        t.s_flag[2] = sk1;
+        t.s_src[0] = sk0;  // read by the source epilogue, after the barrier below
+        t.s_src[1] = sk1;
     }
     __syncthreads();
-    if (tid == 0)  // planes ktop .. ktop-3 into slots 0..3
-        for (int p = ktop, q = 0; q < RING && p >= klow; p--, q++) {
-            // the air plane (k = -1) is the boundary's output: a top chunk launched early (programmatic
-            // dependent launch after the boundary's last stage) stages its other planes first
-            if (p < 0) pdl_wait_prev();
-            uint64_t *b = t.bars + q;
-            mbar_expect_tx(b, t.plane_bytes);
-            for (int a = 0; a < NARR; a++) tma_load_3d(t.ring + (q * NARR + a) * BS, t.maps + a, t.i0, t.j0, p + 1, b);
-        }
+    if (t.duty == 1) {  // B and sigma of plane ktop through slot 3, stages ktop .. ktop-2 into slots 0..2
+        uint64_t *b = t.bars + 3;
+        mbar_expect_tx(b, (unsigned)(3 * BOX * sizeof(T)));
+        for (int a : {ABX, ABY, ASG})
+            tma_load_3d(t.sm + (3 * NARR + a) * BS, maps.m + a, t.i0, t.j0, ktop + 1, b);
+        for (int q = 0; q < 3 && ktop - q >= t.k0; q++) load_stage(t, ktop - q, q);
+    }
     // chunk offsets of Bz over the box (zero without chunking)
     for (int e = tid; e < BOX; e += NT) {
         T o = T(0), o1 = T(0);
@@ -432,8 +465,8 @@ __device__ __forceinline__ void sweep_cta(const SweepMaps &maps, const Geom &g, 
                 T pv[kMaxChunks];  // all loads in flight together
 #pragma unroll
                 for (int q = 1; q < kMaxChunks; q++)
-                    pv[q] = q > c && q < zc.n && TCSEM_IN(q * t.PS + pc, zc.n * t.PS, err) ? ld_in<FRESH>(tin + q * t.PS + pc) : T(0);
-                const T first = c + 1 < zc.n ? ld_in<FRESH>(tin + (c + 1) * t.PS + pc) : T(0);
+                    pv[q] = q > c && q < zc.n && TCSEM_IN(q * PS + pc, zc.n * PS, err) ? ld_in<FRESH>(tin + q * PS + pc) : T(0);
+                const T first = c + 1 < zc.n ? ld_in<FRESH>(tin + (c + 1) * PS + pc) : T(0);
 #pragma unroll
                 for (int q = 1; q < kMaxChunks; q++)
                     if (q > c && q < zc.n) o += pv[q];
@@ -443,54 +476,54 @@ __device__ __forceinline__ void sweep_cta(const SweepMaps &maps, const Geom &g, 
         s_oc[e] = o;
         s_oc1[e] = o1;
     }
-    {  // every thread observes the completion of the first two planes
-        bool ok = mbar_wait_bounded(t.bars + 0, 0u);
-        ok = ok && mbar_wait_bounded(t.bars + 1, 0u);
-        if (!ok) *t.s_flag = 1;
-    }
+    t.bad = !mbar_wait_bounded(t.bars + 3, 0u);
+    if (!t.bad) t.bad = !mbar_wait_bounded(t.bars + 0, 0u);
+    carry_plane(t, t.sm + 3 * NARR * BS);
+    t.ex1 = t.ey1 = t.exn = t.eyn = t.ezn = dup<T>(T(0));
+    t.bxo1 = t.byo1 = t.bxn = t.byn = t.acc = dup<T>(T(0));
+    async_shared_fence();
     __syncthreads();
-    if (*t.s_flag) {  // record it, let the first planes land, leave together
-        if (tid == 0) {
-            atomicExch(err, 1);
-            for (int q = 0; q < RING && ktop - q >= klow; q++) mbar_wait_bounded(t.bars + q, 0u);
-        }
-        return;
-    }
-#pragma unroll
-    for (int q = 0; q < NC; q++) {
-        const int so = t.so[q];
-        const T *p0 = t.ring + so;  // carried values of plane ktop (slot 0)
-        const T a = p0[ASG * BS], b = p0[ASG * BS - 1], cc = p0[ASG * BS - BXW], d = p0[ASG * BS - BXW - 1];
-        t.sxk[q] = a + cc;
-        t.syk[q] = a + b;
-        t.szk[q] = a + cc + b + d;
-        t.bxk[q] = p0[ABX * BS];
-        t.byk[q] = p0[ABY * BS];
-        t.ex1[q] = t.ey1[q] = t.exn[q] = t.eyn[q] = t.ezn[q] = T(0);
-        t.bxo1[q] = t.byo1[q] = t.bxn[q] = t.byn[q] = t.acc[q] = T(0);
-    }
+    if (t.duty == 1 && ktop - 3 >= t.k0) load_stage(t, ktop - 3, 3);
 
     // Bz offsets of the first plane: ktop is the halo plane k1 of the chunk below (its offsets) or the
     // zero bottom; every later plane lies in this chunk
     set_offsets(t, ktop < N ? s_oc1 : s_oc);
     // FP64 (bound by the FP64 pipe): the halo warps run their reduced copies of the plane code
-    // (5 % faster).  FP32 runs one copy in every warp: three copies of its issue-bound loop made the
-    // sweep 40 % slower (measured; presumably the larger loop no longer fits the instruction cache).
-    bool ok;
-    if constexpr (sizeof(T) == 8)
-        ok = t.role == 0 ? sweep_march<T, 0>(t, s, s_z, out, src, src_tile, s_oc)
-             : t.role == 1 ? sweep_march<T, 1>(t, s, s_z, out, src, src_tile, s_oc)
-                           : sweep_march<T, 2>(t, s, s_z, out, src, src_tile, s_oc);
-    else
-        ok = sweep_march<T, 0>(t, s, s_z, out, src, src_tile, s_oc);
-    if (!ok) {  // a copy did not arrive (the copies in flight were drained in sweep_plane)
-        if (tid == 0) atomicExch(err, 1);
+    // (5 % faster).  FP32 runs one copy in every warp: three copies of its loop made the sweep 40 %
+    // slower (measured; presumably the larger loop no longer fits the instruction cache).
+    if constexpr (sizeof(T) == 8) {
+        if (t.role == 0) sweep_march<T, 0>(t, s, s_z, src, s_oc);
+        else if (t.role == 1) sweep_march<T, 1>(t, s, s_z, src, s_oc);
+        else sweep_march<T, 2>(t, s, s_z, src, s_oc);
+    } else {
+        sweep_march<T, 0>(t, s, s_z, src, s_oc);
+    }
+    // the last plane's Bz, in the buffer of its parity
+    async_shared_fence();
+    const bool bad = __syncthreads_or(t.bad);
+    if (t.duty == 2) {
+        tma_store_3d(maps.o + 5, t.sm + ((ktop - klow) & 1 ? soff<T>(SBZ, 1) : soff<T>(SBZ, 0)), t.i0, t.j0, t.k0);
+        bulk_commit();
+        bulk_wait_all();
+    }
+    if (bad) {  // a copy did not arrive: record it and let the last planes land
+        if (t.duty == 1) {
+            atomicExch(err, 1);
+            for (int k = t.k0; k <= ktop && k < t.k0 + RING; k++) {
+                const int n = ktop - k;  // stages land in order: slot n % RING, round n / RING
+                mbar_wait_bounded(t.bars + n % RING, (unsigned)(n / RING + (n % RING == 3)) & 1u);
+            }
+        }
+        __syncthreads();
         return;
     }
-    if (zc.n > 1) {
+    if (zc.n > 1 && t.role == 0) {
+        const T a[2] = {t.acc.a, t.acc.b};
 #pragma unroll
-        for (int q = 0; q < NC; q++)
-            if (t.own[q] && TCSEM_IN(c * t.PS + t.col[q], zc.n * t.PS, err)) tout[c * t.PS + t.col[q]] = t.acc[q];
+        for (int q = 0; q < 2; q++) {
+            const int o = c * PS + (t.j + 1) * XP + t.i + 32 * q + 4;
+            if (t.j < M && t.i + 32 * q < L && TCSEM_IN(o, zc.n * PS, err)) tout[o] = a[q];
+        }
     }
 }
 

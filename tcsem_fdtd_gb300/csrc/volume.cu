@@ -126,8 +126,8 @@ void launch_bderivate(const Geom &g, FieldSet<T> f, const Axis<T> &ax, T dtb, in
 
 template <typename T>
 __global__ void __launch_bounds__(fs3::NT, sizeof(T) == 4 ? 2 : 1)
-    k_sweep(const __grid_constant__ SweepMaps maps, Geom g, FieldSet<T> out, const T *__restrict__ tin,
-            T *__restrict__ tout, Axis<T> ax, StepScalars<T> sdir, const StepScalars<T> *__restrict__ table,
+    k_sweep(const __grid_constant__ SweepMaps maps, Geom g, const T *__restrict__ tin, T *__restrict__ tout,
+            Axis<T> ax, StepScalars<T> sdir, const StepScalars<T> *__restrict__ table,
             StepGate gate, SourceTable<T> src, ZChunks zc, int cbase, int rev, int *err) {
     StepScalars<T> s = sdir;
     if (gate.base) {
@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(fs3::NT, sizeof(T) == 4 ? 2 : 1)
         s = table[st];
     }
     const int c = cbase + (int)(rev ? gridDim.z - 1 - blockIdx.z : blockIdx.z);
-    sweep_cta<T>(maps, g, out, tin, tout, ax, s, src, zc, blockIdx.x, blockIdx.y, c, err);
+    sweep_cta<T>(maps, g, tin, tout, ax, s, src, zc, blockIdx.x, blockIdx.y, c, err);
 }
 
 // every slot of a batch in one launch: block b belongs to the slot whose range of idx holds it
@@ -149,12 +149,12 @@ __global__ void __launch_bounds__(fs3::NT, sizeof(T) == 4 ? 2 : 1)
     if (st >= d.nsteps) return;
     const int lb = blockIdx.x - idx.off[q];
     const int bx = lb % d.tiles_x, rest = lb / d.tiles_x, by = rest % d.tiles_y, c = c0 + rest / d.tiles_y;
-    sweep_cta<T>(d.maps, d.g, d.out, d.tin, d.tout, d.ax, d.table[st], d.src, d.zc, bx, by, c, d.err);
+    sweep_cta<T>(d.maps, d.g, d.tin, d.tout, d.ax, d.table[st], d.src, d.zc, bx, by, c, d.err);
 }
 
 template <typename T>
-void launch_fused_sweep(const SweepMaps &maps, const Geom &g, FieldSet<T> out, const T *tin, T *tout,
-                        const Axis<T> &ax, StepScalars<T> s, const StepScalars<T> *table, StepGate gate,
+void launch_fused_sweep(const SweepMaps &maps, const Geom &g, const T *tin, T *tout, const Axis<T> &ax,
+                        StepScalars<T> s, const StepScalars<T> *table, StepGate gate,
                         const SourceTable<T> &src, const ZChunks &zc, int c0, int c1, bool rev, int *err,
                         cudaStream_t st, bool pdl) {
     cudaLaunchConfig_t cfg = {};
@@ -167,7 +167,7 @@ void launch_fused_sweep(const SweepMaps &maps, const Geom &g, FieldSet<T> out, c
     at[0].val.programmaticStreamSerializationAllowed = pdl ? 1 : 0;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, k_sweep<T>, maps, g, out, tin, tout, ax, s, table, gate, src, zc, c0, rev ? 1 : 0, err);
+    cudaLaunchKernelEx(&cfg, k_sweep<T>, maps, g, tin, tout, ax, s, table, gate, src, zc, c0, rev ? 1 : 0, err);
 }
 
 template <typename T>
@@ -193,6 +193,8 @@ template <typename T> int sweep_blocks_per_sm(int N) {
 }
 int sweep_box_x() { return fs3::BXW; }
 int sweep_box_y() { return fs3::BYH; }
+int sweep_tile_x() { return fs3::TX; }
+int sweep_tile_y() { return fs3::BY; }
 
 // materialise Bz = P + O_c in place and clear the chunk totals
 template <typename T>
@@ -219,7 +221,7 @@ template <typename T> void launch_bz_consolidate(const Geom &g, T *bz, T *tot, c
     template void launch_update_e<T>(const Geom &, FieldSet<T>, const T *, const Axis<T> &, StepScalars<T>,        \
                                      const SourceTable<T> &, int *, cudaStream_t);                                 \
     template void launch_bderivate<T>(const Geom &, FieldSet<T>, const Axis<T> &, T, int *, cudaStream_t);         \
-    template void launch_fused_sweep<T>(const SweepMaps &, const Geom &, FieldSet<T>, const T *, T *,             \
+    template void launch_fused_sweep<T>(const SweepMaps &, const Geom &, const T *, T *,                          \
                                         const Axis<T> &, StepScalars<T>, const StepScalars<T> *, StepGate,         \
                                         const SourceTable<T> &, const ZChunks &, int, int, bool, int *, cudaStream_t,  \
                                         bool);                                                                     \
