@@ -76,11 +76,12 @@ struct StepGate {
     __device__ __forceinline__ long step() const { return (long)*base + off; }
 };
 
-// z-chunks of the fused sweep: chunk c covers planes [kb[c], kb[c+1]); the
+// layout of the fused sweep: tiles of 64 x `rows` columns; chunk c covers planes [kb[c], kb[c+1]); the
 // top chunk may be shorter than the others (it runs after the boundary)
 constexpr int kMaxChunks = 16;
 struct ZChunks {
     int n;
+    int rows;  // rows of a tile of the sweep, at most 8
     int kb[kMaxChunks + 1];
     // kb[c] for a run-time c without indexing the array (it may live in the
     // kernel's parameter space)
@@ -121,7 +122,6 @@ template <typename T> int sweep_blocks_per_sm(int N);  // resident sweep CTAs pe
 int sweep_box_x();
 int sweep_box_y();
 int sweep_tile_x();
-int sweep_tile_y();
 template <typename T> void launch_bz_consolidate(const Geom &g, T *bz, T *tot, const ZChunks &zc, cudaStream_t st);
 
 // ------------------------------------------------------------------ batches
@@ -162,6 +162,6 @@ template <typename T> struct SweepSlot {
 template <typename T>
 void launch_sweep_batched(const SweepSlot<T> *slots, const BatchIndex &idx, int s, int c0, int N_max, cudaStream_t st);
 int sweep_tiles_x(int L);
-int sweep_tiles_y(int M);
+int sweep_tiles_y(int M, int rows);
 
 }  // namespace tcsem

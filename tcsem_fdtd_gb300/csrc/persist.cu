@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(fs3::NT, sizeof(T) == 4 ? 2 : 1) k_persistent(
             // retire the unit's mbarriers before the next unit lays out shared memory anew
             if (bars == 2) {
                 uint64_t *ring = reinterpret_cast<uint64_t *>(smem_raw + fs3::bars_offset<T>());
-                for (int q = 0; q < fs3::RING; q++) mbar_inval(ring + q);
+                for (int q = 0; q < fs3::ring<T>(); q++) mbar_inval(ring + q);
             } else if (bars == 1) {
                 mbar_inval(reinterpret_cast<uint64_t *>(smem_raw));  // offset 0 in every boundary layout
             }

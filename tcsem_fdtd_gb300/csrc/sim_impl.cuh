@@ -173,7 +173,7 @@ struct SimBase {
 template <typename T> struct SimImpl : SimBase {
     Geom g{};
     DevMem fld[2][6], con, tot[2];  // two field sets + conductivity; per-set chunk totals of Bz
-    ZChunks zc{};
+    ZChunks zc{0, 8, {}};
     SweepMaps maps[2];              // TMA descriptors of the sweep that reads each field set
     DevMem errw;                    // device error word (a bounded wait gave up)
     DevMem axis_mem;
@@ -282,9 +282,12 @@ template <typename T> struct SimImpl : SimBase {
             const T *b = axis_mem.as<T>();
             ax = {b + o[0], b + o[1], b + o[2], b + o[3], b + o[4], b + o[5], b + o[6], b + o[7], b + o[8]};
         }
+        errw.alloc(sizeof(int));
+        dev_bytes += sizeof(int);
+        dzero(errw.p, sizeof(int));
+        init_boundary();
         init_chunks();
         init_maps();
-        init_boundary();
         init_steps();
         // the top chunk's air plane is the only input of the sweep that the boundary writes
         overlap = zc.n > 1 && !opts.serial_boundary;
@@ -391,30 +394,54 @@ template <typename T> struct SimImpl : SimBase {
     }
     // most chunks a layout may have: every chunk keeps at least 8 planes
     int max_chunks() const { return std::max(1, std::min(kMaxChunks, model.N / 8)); }
-    // z-chunks of the fused sweep.  Overlapped step: a one-plane top chunk (the only part of
+    // z-chunks (and FP64: tile rows) of the fused sweep.  Overlapped step: a one-plane top chunk (the only part of
     // the sweep that waits for the boundary) and lower chunks whose CTAs fit in one wave;
     // deeper chunks also mean fewer halo planes.  In FP32 the sweep is bound by memory and
-    // the wave leaves about 15 % of the CTA slots to the boundary kernels running beside it;
-    // in FP64 it is bound by the FP64 pipes and the wave fills the slots as far as it can.
+    // the wave leaves about 15 % of the CTA slots to the boundary kernels running beside it.
     // Serial step: enough CTAs to fill the GPU several times over, split evenly.
     void init_chunks() {
         const Model &m = model;
         int sms = 0;
         CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
         CK(sweep_configure<T>(m.N));
-        const long tiles = (long)sweep_tiles_x(m.L) * sweep_tiles_y(m.M);
-        const long slots = (long)sms * sweep_blocks_per_sm<T>(m.N);
-        int n, top = 0;
+        const int per_sm = sweep_blocks_per_sm<T>(m.N);
+        const long slots = (long)sms * per_sm;
+        long tiles = (long)sweep_tiles_x(m.L) * sweep_tiles_y(m.M, zc.rows);
+        int n, top = 0, most = max_chunks();
         if (opts.serial_boundary) {
             n = (int)std::min<long>(kMaxChunks, std::max<long>(1, (7L * sms + tiles - 1) / tiles));
+        } else if (sizeof(T) == 8) {
+            // The FP64 pipes bound both branches of the step, and a boundary block beside a sweep CTA takes
+            // twice as long: the fastest layout gives the lower chunks one wave on some of the SMs and the
+            // boundary the others.  Estimated times in us, of all tile heights and chunk counts: a sweep CTA
+            // costs its rows and one more (halo) times its planes and 1.25 more; the boundary's operations
+            // run at two lanes per clock on the SMs left free, after about 25 us of latency, or after the sweep.
+            // Measured, us per step with this rule and with 8 rows and one chunk more than 85 % of the SMs hold
+            // (chunks of 8 planes or more): 44 x 38 x 27 49 and 145, 64 x 64 x 48 78 and 116, 160 x 56 x 40 131 and
+            // 139, 128 x 128 x 96 228 and 265, 187 x 121 x 101 386 and 594, 256 x 256 x 160 1349 and 1583.
+            const double work = (((m.M + 1) / 2 + bd.S) * fft_ops(bd.px) + 3.0 * bd.H * fft_ops(bd.py)) / 4140.0;
+            double best = 1e30;
+            int lower = 1;
+            for (int r = 8; r >= 3; r--) {
+                const long tl = (long)sweep_tiles_x(m.L) * sweep_tiles_y(m.M, r);
+                for (int q = 1; q < kMaxChunks && (q == 1 || (m.N - 1) / q >= 2); q++) {
+                    const long waves = (tl * q + slots - 1) / slots, left = slots - tl * q;
+                    const double low = 4 + waves * 0.95 * (r + 1) * ((m.N - 1 + q - 1) / q + 1.25),
+                                 last = 4 + 0.95 * (r + 1) * 3 * ((tl + slots - 1) / slots),
+                                 beside = left > 0 ? std::max(low, 25 + work / left + last) : 1e30,
+                                 after = low + 40 + work / slots + last;
+                    if (std::min(beside, after) < 0.99 * best) best = std::min(beside, after), zc.rows = r, lower = q;
+                }
+            }
+            if (opts.zchunks > 0) zc.rows = 8;
+            n = 1 + lower;
+            top = 1;
+            most = kMaxChunks;
         } else {
-            const long want = slots * 85 / 100;
-            long lower = std::max<long>(1, want / tiles);
-            if (sizeof(T) == 8 && (lower + 1) * tiles <= slots) lower++;
-            n = 1 + (int)lower;
+            n = 1 + (int)std::max<long>(1, slots * 85 / 100 / tiles);
             top = 1;
         }
-        n = std::min(n, max_chunks());
+        n = std::min(n, most);
         rule_lower = n - 1;
         if (opts.zchunks > 0) n = std::min(std::min(opts.zchunks, kMaxChunks), m.N);
         if (opts.top_planes != 0) top = opts.top_planes;  // > 0: that many planes, < 0: an even split
@@ -438,7 +465,7 @@ template <typename T> struct SimImpl : SimBase {
         const cuuint32_t estr[3] = {1, 1, 1};
         const CUtensorMapDataType dt = sizeof(T) == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
         const cuuint64_t odims[3] = {(cuuint64_t)g.L, (cuuint64_t)g.M, (cuuint64_t)g.N};
-        const cuuint32_t obox[3] = {(cuuint32_t)sweep_tile_x(), (cuuint32_t)sweep_tile_y(), 1};
+        const cuuint32_t obox[3] = {(cuuint32_t)sweep_tile_x(), (cuuint32_t)zc.rows, 1};
         auto make = [&](void *ptr, CUtensorMap *m, const cuuint64_t *dim, const cuuint32_t *bx) {
             CUresult r = enc(m, dt, 3, ptr, dim, strides, bx, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                              CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -452,9 +479,6 @@ template <typename T> struct SimImpl : SimBase {
             }
             make(con.p, &maps[b].m[6], dims, box);
         }
-        errw.alloc(sizeof(int));
-        dev_bytes += sizeof(int);
-        dzero(errw.p, sizeof(int));
         CK(sweep_configure<T>(g.N));
     }
     void check_error() override { check_device_error(); }
@@ -508,6 +532,15 @@ template <typename T> struct SimImpl : SimBase {
         for (int i = 0; i < d; i++) w[i] = 0.5 * (1.0 - std::cos(kPi * i / d));
         for (int i = d + nu; i < n; i++) w[i] = 0.5 * (1.0 - std::cos(kPi * (n - i) / (r + 1)));
         return w;
+    }
+    // operations of the boundary's transforms: of a line of radix stages, c(p) per point and stage
+    static double fft_ops(const FFTPlan &P) {
+        double c = 0;
+        for (int q = 0; q < P.nst; q++) {
+            const int p = P.radix[q];
+            c += p == 2 ? 6 : p == 3 ? 9 : p == 4 ? 8 : p == 5 ? 14 : p == 8 ? 12 : p + 8;
+        }
+        return P.n * c;
     }
     void init_boundary() {
         const Model &m = model;
@@ -844,13 +877,13 @@ template <typename T> struct SimImpl : SimBase {
         sw.maps = maps[b]; sw.g = g; sw.tin = tot[b].as<T>(); sw.tout = tot[b ^ 1].as<T>();
         sw.ax = ax; sw.table = steps.as<StepScalars<T>>(); sw.step_base = counter; sw.nsteps = sched.nsteps;
         sw.src = src; sw.zc = zc; sw.err = errw.as<int>();
-        sw.tiles_x = sweep_tiles_x(g.L); sw.tiles_y = sweep_tiles_y(g.M);
+        sw.tiles_x = sweep_tiles_x(g.L); sw.tiles_y = sweep_tiles_y(g.M, zc.rows);
         bs.bd = bd; bs.g = g; bs.bz = in.bz; bs.tot = tot[b].as<T>(); bs.nch = zc.n; bs.bx = in.bx; bs.by = in.by;
         bs.step_base = counter; bs.nsteps = sched.nsteps;
         rs.rd = rd; rs.f = out; rs.tot = tot[b ^ 1].as<T>(); rs.zc = zc; rs.g = g;
         rs.step_base = counter; rs.nsteps = sched.nsteps;
     }
-    int sweep_blocks() const { return sweep_tiles_x(g.L) * sweep_tiles_y(g.M) * zc.n; }
+    int sweep_blocks() const { return sweep_tiles_x(g.L) * sweep_tiles_y(g.M, zc.rows) * zc.n; }
     int rx_stencils() const { return rd.NComp * rd.nr; }
     // an upper bound of the device memory init() allocates, from the host model alone
     static size_t estimate_bytes(const Model &m, long nsteps, int padded_plane) {
@@ -1023,6 +1056,27 @@ template <typename T> struct SimImpl : SimBase {
         ok = (std::fclose(f) == 0) && ok;
         if (!ok) throw Error(TCSEM_ERR_IO, std::string("cannot write ") + path);
     }
+    int earlier_chunks() const {
+        int sms = 0;
+        CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+        const long tiles = (long)sweep_tiles_x(model.L) * sweep_tiles_y(model.M, 8);
+        long lower = std::max<long>(1, sms * 85L / 100 / tiles);
+        if ((lower + 1) * tiles <= sms) lower++;
+        return (int)std::min<long>(1 + lower, max_chunks());
+    }
+    void adopt_layout(const ZChunks &lay) {
+        CK(cudaStreamSynchronize(stream));
+        zc = lay;
+        for (auto &e : gexec) if (e) { cudaGraphExecDestroy(e); e = nullptr; }
+        const size_t tb = (size_t)zc.n * g.PS * sizeof(T);
+        for (int b = 0; b < 2 && tot[b].n < tb; b++) {
+            dev_bytes += tb - tot[b].n;
+            tot[b].alloc(tb);
+        }
+        overlap = overlap && zc.n > 1;
+        chunks_used = zc.n;
+        top_used = overlap ? zc.kb[1] : 0;
+    }
     // into a handle of the same survey, precision and z-chunk layout; the run continues with advance
     void load_state(const char *path) override {
         std::FILE *f = std::fopen(path, "rb");
@@ -1035,17 +1089,27 @@ template <typename T> struct SimImpl : SimBase {
             throw Error(st, m);
         };
         if (!ok || std::memcmp(h.magic, "TCSEMST", 8) != 0 || h.version != 2) fail(TCSEM_ERR_PARSE, std::string(path) + " is not a saved run state");
-        bool same = h.tsize == (int)sizeof(T) && h.L == model.L && h.M == model.M && h.N == model.N && h.nch == zc.n &&
-                    h.field_bytes == (long long)fld[0][0].n && h.tot_bytes == (long long)zc.n * g.PS * (long long)sizeof(T) &&
+        // a handle with the default layout also continues a state saved in the layout that was the default before
+        // the tile heights and chunk counts were chosen together
+        ZChunks lay = zc;
+        if (sizeof(T) == 8 && ok && opts.zchunks == 0 && opts.top_planes == 0 && !opts.serial_boundary && h.nch != zc.n) {
+            const ZChunks now = zc;
+            set_chunks(earlier_chunks(), 1);
+            lay = zc;
+            zc = now;
+        }
+        bool same = h.tsize == (int)sizeof(T) && h.L == model.L && h.M == model.M && h.N == model.N && h.nch == lay.n &&
+                    h.field_bytes == (long long)fld[0][0].n && h.tot_bytes == (long long)lay.n * g.PS * (long long)sizeof(T) &&
                     (h.cur == 0 || h.cur == 1) && h.step >= 0 && h.step <= sched.nsteps && h.itx >= 0 &&
                     h.itx < (int)model.in.tx.size() && h.L1 == model.L1 && h.M1 == model.M1 &&
                     h.padded_plane == opts.padded_plane && h.fix_dual_bipole == (opts.fix_dual_bipole != 0) &&
                     h.nsteps == sched.nsteps;
-        for (int c = 0; c <= zc.n && same; c++) same = h.kb[c] == zc.kb[c];
+        for (int c = 0; c <= lay.n && same; c++) same = h.kb[c] == lay.kb[c];
         const std::string other = std::string(path) + " was saved by a different survey, precision, z-chunk layout, "
                                                       "continuation plane or dual-bipole option";
         if (!same) fail(TCSEM_ERR_INVALID, other);
         try {
+            if (lay.n != zc.n) adopt_layout(lay);
             begin(h.itx);  // the transmitter's tables (receiver buffers) and a zero state, then the saved arrays
             // the zeroing runs on the handle's (non-blocking) stream: let it finish before the copies
             CK(cudaStreamSynchronize(stream));

@@ -48,7 +48,10 @@ constexpr int BOX = BXW * BYH;
 constexpr int NARR = 7;                // ex ey ez bx by bz sigma
 // ring stride of one box: rounded up to 128 bytes so every TMA destination is 128-byte aligned
 template <typename T> __host__ __device__ constexpr int boxs() { return (int)(((BOX * sizeof(T) + 127) / 128) * 128 / sizeof(T)); }
-constexpr int RING = 4;                // stages in flight
+// stages in flight: four in FP32, where two CTAs share an SM and memory is the bound; two in FP64, where a
+// plane takes several times a copy's latency on the FP64 pipe, which leaves room for boundary blocks beside
+// the one CTA of an SM
+template <typename T> __host__ __device__ constexpr int ring() { return sizeof(T) == 4 ? 4 : 2; }
 enum { AEX = 0, AEY, AEZ, ABX, ABY, ABZ, ASG };
 // New planes in shared memory, two buffers each.  Those that neighbours read (Ez, Bx, By): nine dense rows
 // of 64 (the ninth is the +y halo row), then the +x halo column, then cells nobody reads for idle
@@ -56,11 +59,11 @@ enum { AEX = 0, AEY, AEZ, ABX, ABY, ABZ, ASG };
 constexpr int XCOL = 9 * TX, XBUF = 10 * TX, SBUF = BY * TX;
 enum { XEZ = 0, XBX, XBY };
 enum { SEX = 0, SEY, SBZ };
-template <typename T> __host__ __device__ constexpr int xoff(int a, int q) { return RING * NARR * boxs<T>() + (2 * a + q) * XBUF; }
+template <typename T> __host__ __device__ constexpr int xoff(int a, int q) { return ring<T>() * NARR * boxs<T>() + (2 * a + q) * XBUF; }
 template <typename T> __host__ __device__ constexpr int soff(int a, int q) { return xoff<T>(3, 0) + (3 * q + a) * SBUF; }
-// byte offset of the RING mbarriers, the error flag and source planes, then the z tables
+// byte offset of the ring's mbarriers and the source planes; then the z tables
 template <typename T> __host__ __device__ constexpr size_t bars_offset() { return (size_t)soff<T>(0, 2) * sizeof(T); }
-template <typename T> __host__ __device__ constexpr size_t smem_bytes() { return bars_offset<T>() + RING * 8 + 16; }
+template <typename T> __host__ __device__ constexpr size_t smem_bytes() { return bars_offset<T>() + ring<T>() * 8 + 16; }
 template <typename T> size_t smem_bytes_n(int N) {  // plus the z tables
     return smem_bytes<T>() + 3 * (size_t)(N + 3) * 2 * sizeof(T);
 }
@@ -69,29 +72,22 @@ template <typename T> size_t smem_bytes_n(int N) {  // plus the z tables
 static_assert(2 * BOX <= 3 * SBUF, "the offset boxes fit the first store buffers");
 }  // namespace fs3
 
-// reciprocal used by the E update: one MUFU op in FP32 (about 1 ulp), exact division in FP64
-template <typename T> __device__ __forceinline__ T rcp_fast(T x);
-template <> __device__ __forceinline__ float rcp_fast<float>(float x) {
+// reciprocals of the E update: one MUFU op in FP32 (about 1 ulp)
+__device__ __forceinline__ float rcp_fast(float x) {
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
-template <> __device__ __forceinline__ double rcp_fast<double>(double x) { return 1.0 / x; }
-
-// the three reciprocals of the E update: three MUFU ops in FP32; in FP64, where a division
-// costs about ten FP64 pipe operations and the pipe bounds the sweep, one division of the
-// product and five multiplies (1/a = bc / abc, ...), a few ulp from three divisions
-__device__ __forceinline__ void recip3(float a, float b, float c, float &ra, float &rb, float &rc) {
-    ra = rcp_fast(a);
-    rb = rcp_fast(b);
-    rc = rcp_fast(c);
+// In FP64 the hardware's approximation r0 of 1/x (a MUFU op, about 20 bits) and one third-order step of
+// Householder's iteration, 1/x = r0 / (1 - e) = r0 (1 + e + e^2 + ...) with e = 1 - x r0: what is left out is
+// e^3 ~ 2^-60, and three FP64 operations take the place of a division's (normal x only)
+__device__ __forceinline__ double rcp64(double x) {
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+    const double e = ::fma(-x, r, 1.0);
+    return ::fma(r, ::fma(e, e, e), r);
 }
-__device__ __forceinline__ void recip3(double a, double b, double c, double &ra, double &rb, double &rc) {
-    const double ab = a * b, r = 1.0 / (ab * c), rab = c * r;
-    rc = ab * r;
-    ra = b * rab;
-    rb = a * rab;
-}
+__device__ __forceinline__ Pair<double> rcp64(Pair<double> x) { return {rcp64(x.a), rcp64(x.b)}; }
 
 // per-thread state of the sweep; sweep_plane<PH>() advances one z-plane with PH = (ktop - k) mod 4, so ring
 // slots and buffer parities are compile-time constants
@@ -101,8 +97,8 @@ template <typename T> struct SweepThread {
     int *s_src;  // first and last plane with a source segment in the tile
     const SweepMaps *maps;
     int j, N, k0, k1, klow, ktop, i0, j0;
-    int role;     // 0: a row of the tile, 1: the +y halo row, 2: the +x halo column (warp-uniform)
-    int duty;     // 1: the thread issues the loads (a lane of the +y warp), 2: the stores (of the +x warp)
+    int role;     // 0: a row of the tile, 1: the +y halo row, 2: the +x halo column, 3: none (warp-uniform)
+    int duty;     // 1: the thread issues the loads (a lane of warp 8), 2: the stores (of the +x warp)
     bool bad;     // a copy did not arrive
     bool src;     // a source segment touches the tile in this step
     int so, xo, xd, xr, i;         // first cell: in the box, in the new planes; its +y and the second one's +x neighbour; x index
@@ -111,9 +107,14 @@ template <typename T> struct SweepThread {
     unsigned upd;
     bool edge;
     Pair<T> rdy2, rdy, fy;         // per row: 1/(dy[j-1]+dy[j]), 1/dy[j], dtb/dy[j]
-    Pair<T> lam, c4;               // FP32: 2 lambda / (dt/4), c4 / (dt/4); FP64: 2 lambda, c4
+    // 2 lambda, dt/4 (the sweep forms sigma sums of four cells), c4.  FP64: c4 is in rdx2, rdy2 and the z
+    // table's 1/(dz[k-1]+dz[k]), and t.c4 is 4 lambda
+    Pair<T> lam, dt, c4;
     Pair<T> rdx2, rdx, fx;
-    Pair<T> oc0, oci, ocj;  // Bz chunk offsets of the plane being updated: at, left of, below the cells
+    // Bz chunk offsets of the plane being updated: at, left of, below the cells (FP64: left minus at, at minus
+    // below, and whether there are any)
+    Pair<T> oc0, oci, ocj;
+    bool offsets;
     Pair<T> ex1, ey1, exn, eyn, ezn;
     Pair<T> bxo1, byo1, bxn, byn, acc;
     Pair<T> sxk, syk, szk, bxk, byk, bxj, byi;  // of plane k: sigma sums, own B, Bx below and By left of the cell
@@ -127,21 +128,30 @@ template <typename T> __device__ __forceinline__ void keep(Pair<T> &v, Pair<T> o
 // the thread's two cells at offset o
 template <typename T> __device__ __forceinline__ Pair<T> cells(const T *p, int o) { return pair<T>(p[o], p[o + 32]); }
 template <typename T> __device__ __forceinline__ void put_cells(T *p, int o, Pair<T> v) { p[o] = v.a; p[o + 32] = v.b; }
+// ... of which the +x halo column has one (ROLE 2: the second one's arithmetic is dead code)
+template <int ROLE, typename T> __device__ __forceinline__ Pair<T> rcells(const T *p, int o) {
+    if constexpr (ROLE == 2) return pair<T>(p[o], T(0));
+    else return cells(p, o);
+}
+template <int ROLE, typename T> __device__ __forceinline__ void rput(T *p, int o, Pair<T> v) {
+    if constexpr (ROLE == 2) p[o] = v.a;
+    else put_cells(p, o, v);
+}
 
 // sigma sums and B of the plane in the B and sigma boxes p
-template <typename T> __device__ __forceinline__ void carry_plane(SweepThread<T> &t, const T *p) {
+template <int ROLE, typename T> __device__ __forceinline__ void carry_plane(SweepThread<T> &t, const T *p) {
     using namespace fs3;
     constexpr int BS = boxs<T>();
     const T *sg = p + ASG * BS;
     const int so = t.so;
-    const Pair<T> a = cells(sg, so), b = cells(sg, so - 1), c = cells(sg, so - BXW), d = cells(sg, so - BXW - 1);
+    const Pair<T> a = rcells<ROLE>(sg, so), b = rcells<ROLE>(sg, so - 1), c = rcells<ROLE>(sg, so - BXW), d = rcells<ROLE>(sg, so - BXW - 1);
     t.sxk = a + c;
     t.syk = a + b;
     t.szk = t.sxk + b + d;
-    t.bxk = cells(p + ABX * BS, so);
-    t.byk = cells(p + ABY * BS, so);
-    t.bxj = cells(p + ABX * BS, so - BXW);
-    t.byi = cells(p + ABY * BS, so - 1);
+    t.bxk = rcells<ROLE>(p + ABX * BS, so);
+    t.byk = rcells<ROLE>(p + ABY * BS, so);
+    t.bxj = rcells<ROLE>(p + ABX * BS, so - BXW);
+    t.byi = rcells<ROLE>(p + ABY * BS, so - 1);
 }
 // the loading thread: stage k into slot q
 template <typename T> __device__ __forceinline__ void load_stage(const SweepThread<T> &t, int k, int q) {
@@ -172,9 +182,9 @@ __device__ __forceinline__ void sweep_plane(SweepThread<T> &t, int k, unsigned r
                                             const Pair<T> *zt, const SourceTable<T> &src) {
     using namespace fs3;
     typedef Pair<T> P;
-    constexpr int BS = boxs<T>();
+    constexpr int BS = boxs<T>(), RING = ring<T>();
     constexpr int QE = PH & 1, QB = (PH + 1) & 1;
-    constexpr bool doB = KIND == INNER || KIND == LAST, doE = KIND != LAST;
+    constexpr bool doB = (KIND == INNER || KIND == LAST) && ROLE != 3, doE = KIND != LAST && ROLE != 3;
     zt += 3 * (k - t.klow);  // dtb/dz, 1/(dz[k-1]+dz[k]), dz of plane k
     // Roles (one compiled copy each, FP64 only): the row warps update and store every component; the
     // +y halo row warp only produces what the tile's last row reads from it (Ex and Ez for By there,
@@ -188,7 +198,7 @@ __device__ __forceinline__ void sweep_plane(SweepThread<T> &t, int k, unsigned r
         const P fz = zt[3];
         const T *ez = sm + xoff<T>(XEZ, QB);
         if constexpr (rY) {
-            const P ezj = cells(ez, t.xd);
+            const P ezj = rcells<ROLE>(ez, t.xd);
             t.bxn = fma(t.ezn - ezj, t.fy, fma(t.ey1 - t.eyn, fz, t.bxo1));
         }
         if constexpr (rX) {
@@ -204,44 +214,48 @@ __device__ __forceinline__ void sweep_plane(SweepThread<T> &t, int k, unsigned r
     if constexpr (doE) {
         t.ex1 = t.exn;
         t.ey1 = t.eyn;
-        const T *p0 = sm + PH * NARR * BS;
+        const T *p0 = sm + PH % RING * NARR * BS;
         const int so = t.so;
         const P sx0 = t.sxk, sy0 = t.syk, sz0 = t.szk, bx0 = t.bxk, by0 = t.byk, bxj = t.bxj, byi = t.byi;
-        carry_plane(t, p0);  // plane k-1, the next one up
-        const P ezo = cells(p0 + AEZ * BS, so);
+        carry_plane<ROLE>(t, p0);  // plane k-1, the next one up
+        const P ezo = rcells<ROLE>(p0 + AEZ * BS, so);
         P exo = dup<T>(T(0)), eyo = exo;
-        if constexpr (rX) exo = cells(p0 + AEX * BS, so);
-        if constexpr (rY) eyo = cells(p0 + AEY * BS, so);
+        if constexpr (rX) exo = rcells<ROLE>(p0 + AEX * BS, so);
+        if constexpr (rY) eyo = rcells<ROLE>(p0 + AEY * BS, so);
         if (KIND != FIRST || k < t.N) {
-            const P bz = cells(p0 + ABZ * BS, so) + t.oc0;
+            const P bz = rcells<ROLE>(p0 + ABZ * BS, so);
             // DuFort-Frankel update (ElectricalFiled.cu:89-345) of the three components, computed for
             // every cell and kept where the component is updated; s.dt carries the 1/4 of the sigma sums
-            const P sx = sx0 + t.sxk, sy = sy0 + t.syk, lam = t.lam, c4 = t.c4, rdy2 = t.rdy2, rz2 = zt[1];
-            const P cz = fma(by0 - byi, t.rdx2, -((bx0 - bxj) * rdy2));
-            P cx, cy;
-            if constexpr (rX) cx = fma(bz - (cells(p0 + ABZ * BS, so - BXW) + t.ocj), rdy2, -((by0 - t.byk) * rz2));
-            if constexpr (rY) cy = fma(bx0 - t.bxk, rz2, -((bz - (cells(p0 + ABZ * BS, so - 1) + t.oci)) * t.rdx2));
+            const P sx = sx0 + t.sxk, sy = sy0 + t.syk, lam = t.lam, dt = t.dt, c4 = t.c4, rdy2 = t.rdy2, rz2 = zt[1];
             if constexpr (sizeof(T) == 8) {
-                const P dt = dup<T>(s.dt), Dx = fma(sx, dt, lam), Dy = fma(sy, dt, lam), Dz = fma(sz0, dt, lam);
-                // FP64, bound by the FP64 pipe: with D = lam2 + sigma dt, the update
-                // (lam2 - sigma dt)/D E + c4/D curl is written (2 lam2 E + c4 curl)/D - E -- three
-                // operations per component after 1/D instead of five.  (In FP32, where 1/D is an
-                // approximate reciprocal, the same form raised the trace error of a long whole run on
-                // 142 x 36 x 25 cells to 1.02 % of its peak, and saved 0.3 % of the step time.)
-                P rx, ry, rz;
-                recip3(Dx.a, Dy.a, Dz.a, rx.a, ry.a, rz.a);
-                recip3(Dx.b, Dy.b, Dz.b, rx.b, ry.b, rz.b);
-                const P l2 = lam + lam;
-                if constexpr (rX) t.exn = fma(fma(c4, cx, l2 * exo), rx, -exo);
-                if constexpr (rY) t.eyn = fma(fma(c4, cy, l2 * eyo), ry, -eyo);
-                t.ezn = fma(fma(c4, cz, l2 * ezo), rz, -ezo);
+                // FP64, bound by the FP64 pipe (two lanes per clock and SM): with D = lam2 + sigma dt the
+                // update (lam2 - sigma dt)/D E + c4/D curl is (2 lam2 E + c4 curl)/D - E, with c4 in the
+                // cell sizes of the curl.  (In FP32, where 1/D is an approximate reciprocal, such a form
+                // raised the trace error of a long whole run on 142 x 36 x 25 cells to 1.02 % of its peak.)
+                const P rx = rcp64(fma(sx, dt, lam)), ry = rcp64(fma(sy, dt, lam)), rz = rcp64(fma(sz0, dt, lam));
+                const P l2 = t.c4;
+                if constexpr (rX) {
+                    P db = bz - rcells<ROLE>(p0 + ABZ * BS, so - BXW);
+                    if (t.offsets) db = db + t.ocj;
+                    t.exn = fma(fma(db, rdy2, fma(t.byk - by0, rz2, l2 * exo)), rx, -exo);
+                }
+                if constexpr (rY) {
+                    P db = rcells<ROLE>(p0 + ABZ * BS, so - 1) - bz;
+                    if (t.offsets) db = db + t.oci;
+                    t.eyn = fma(fma(db, t.rdx2, fma(bx0 - t.bxk, rz2, l2 * eyo)), ry, -eyo);
+                }
+                t.ezn = fma(fma(by0 - byi, t.rdx2, fma(bxj - bx0, rdy2, l2 * ezo)), rz, -ezo);
             } else {
+                const P bzo = bz + t.oc0;
+                const P cz = fma(by0 - byi, t.rdx2, -((bx0 - bxj) * rdy2));
+                const P cx = fma(bzo - (rcells<ROLE>(p0 + ABZ * BS, so - BXW) + t.ocj), rdy2, -((by0 - t.byk) * rz2));
+                const P cy = fma(bx0 - t.bxk, rz2, -((bzo - (rcells<ROLE>(p0 + ABZ * BS, so - 1) + t.oci)) * t.rdx2));
                 auto rcp = [](P d) { return pair<T>(rcp_fast(d.a), rcp_fast(d.b)); };
-                // numerator and denominator divided by dt/4: no product with dt per cell
-                const P rx = rcp(lam + sx), ry = rcp(lam + sy), rz = rcp(lam + sz0);
-                t.exn = fma((lam - sx) * rx, exo, (c4 * rx) * cx);
-                t.eyn = fma((lam - sy) * ry, eyo, (c4 * ry) * cy);
-                t.ezn = fma((lam - sz0) * rz, ezo, (c4 * rz) * cz);
+                const P Dx = fma(sx, dt, lam), Dy = fma(sy, dt, lam), Dz = fma(sz0, dt, lam);
+                const P rx = rcp(Dx), ry = rcp(Dy), rz = rcp(Dz), ndt = -dt;
+                t.exn = fma(fma(sx, ndt, lam) * rx, exo, (c4 * rx) * cx);
+                t.eyn = fma(fma(sy, ndt, lam) * ry, eyo, (c4 * ry) * cy);
+                t.ezn = fma(fma(sz0, ndt, lam) * rz, ezo, (c4 * rz) * cz);
             }
             if (t.edge) {
                 if constexpr (rX) keep(t.exn, exo, t.upd);
@@ -277,20 +291,21 @@ __device__ __forceinline__ void sweep_plane(SweepThread<T> &t, int k, unsigned r
         }
         t.bxo1 = bx0;  // B_old(k) for the next plane's B update
         t.byo1 = by0;
-        put_cells(sm + xoff<T>(XEZ, QE), t.xo, t.ezn);  // publish Ez_new(k)
+        rput<ROLE>(sm + xoff<T>(XEZ, QE), t.xo, t.ezn);  // publish Ez_new(k)
         if (KIND != FIRST && rows) {
-            put_cells(sm + soff<T>(SEX, QE), t.xo, t.exn);
-            put_cells(sm + soff<T>(SEY, QE), t.xo, t.eyn);
+            rput<ROLE>(sm + soff<T>(SEX, QE), t.xo, t.exn);
+            rput<ROLE>(sm + soff<T>(SEY, QE), t.xo, t.eyn);
         }
     }
     if constexpr (doB) {  // publish B_new(k+1): Bx where Bz reads it (rows, +x column), By likewise (rows, +y row)
-        if constexpr (rY) put_cells(sm + xoff<T>(XBX, QB), t.xo, t.bxn);
-        if constexpr (rX) put_cells(sm + xoff<T>(XBY, QB), t.xo, t.byn);
+        if constexpr (rY) rput<ROLE>(sm + xoff<T>(XBX, QB), t.xo, t.bxn);
+        if constexpr (rX) rput<ROLE>(sm + xoff<T>(XBY, QB), t.xo, t.byn);
     }
-    // stage k-1 is read by the next plane; a thread whose wait gave up does not wait again.  Slot 3 is one
-    // phase ahead: it carried plane ktop's B and sigma first.
-    constexpr int NS = (PH + 1) & 3;
-    if (doE && k > t.k0 && !t.bad) t.bad = !mbar_wait_bounded(t.bars + NS, rp ^ (unsigned)((PH + 1) >> 2) ^ (NS == 3 ? 1u : 0u));
+    // stage k-1 is read by the next plane; a thread whose wait gave up does not wait again.  The last slot is
+    // one phase ahead: it carried plane ktop's B and sigma first.
+    constexpr int NS = (PH + 1) % RING;
+    const unsigned parity = (RING == 4 ? rp ^ (unsigned)((PH + 1) >> 2) : (unsigned)((PH + 1) / RING) & 1u) ^ (NS == RING - 1 ? 1u : 0u);
+    if (KIND != LAST && k > t.k0 && !t.bad) t.bad = !mbar_wait_bounded(t.bars + NS, parity);
     async_shared_fence();  // the new planes are read by the TMA
     if (t.duty == 2) bulk_wait_read();  // ... which is done with the buffers the next plane writes
     __syncthreads();
@@ -301,22 +316,22 @@ __device__ __forceinline__ void sweep_plane(SweepThread<T> &t, int k, unsigned r
                 tma_store_3d(t.maps->o + 1, sm + soff<T>(SEY, QE), t.i0, t.j0, k);
                 tma_store_3d(t.maps->o + 2, sm + xoff<T>(XEZ, QE), t.i0, t.j0, k);
             }
-            if constexpr (doB) {
+            if constexpr (KIND == INNER || KIND == LAST) {
                 tma_store_3d(t.maps->o + 3, sm + xoff<T>(XBX, QB), t.i0, t.j0, k + 1);
                 tma_store_3d(t.maps->o + 4, sm + xoff<T>(XBY, QB), t.i0, t.j0, k + 1);
                 if (k + 2 < t.k1) tma_store_3d(t.maps->o + 5, sm + soff<T>(SBZ, QB), t.i0, t.j0, k + 2);
             }
             bulk_commit();
-        } else if (doE && k - RING >= t.k0) {  // the slot takes stage k-4
-            load_stage(t, k - RING, PH);
+        } else if (KIND != LAST && k - RING >= t.k0) {  // the slot takes the stage RING planes up
+            load_stage(t, k - RING, PH % RING);
         }
     }
     // ---- Bz(k+1) = Bz(k+2) + dz (dBx/dx + dBy/dy), for the tile's own rows
     if (doB && rows) {
         const T *bx = sm + xoff<T>(XBX, QB), *by = sm + xoff<T>(XBY, QB);
-        const P bxr = pair<T>(bx[t.xo + 1], bx[t.xr]), byu = cells(by, t.xd);
+        const P bxr = pair<T>(bx[t.xo + 1], bx[t.xr]), byu = rcells<ROLE>(by, t.xd);
         t.acc = fma(zt[5], fma(bxr - t.bxn, t.rdx, (byu - t.byn) * t.rdy), t.acc);
-        put_cells(sm + soff<T>(SBZ, QE), t.xo, t.acc);
+        rput<ROLE>(sm + soff<T>(SBZ, QE), t.xo, t.acc);
     }
 }
 
@@ -325,6 +340,10 @@ template <typename T> __device__ __forceinline__ void set_offsets(SweepThread<T>
     t.oc0 = cells(box, t.so);
     t.oci = cells(box, t.so - 1);
     t.ocj = cells(box, t.so - fs3::BXW);
+    if (sizeof(T) == 8) {
+        t.oci = t.oci - t.oc0;
+        t.ocj = t.oc0 - t.ocj;
+    }
 }
 
 // the z-march of one warp through the chunk, in the copy of the plane code for its role
@@ -363,7 +382,7 @@ __device__ __forceinline__ void sweep_cta(const SweepMaps &maps, const Geom &g, 
                                           T *__restrict__ tout, const Axis<T> &ax, StepScalars<T> s,
                                           const SourceTable<T> &src, const ZChunks &zc, int bx, int by, int c, int *err) {
     using namespace fs3;
-    constexpr int BS = boxs<T>();
+    constexpr int BS = boxs<T>(), RING = ring<T>();
     extern __shared__ __align__(128) unsigned char smem_raw[];
     SweepThread<T> t;
     t.sm = reinterpret_cast<T *>(smem_raw);
@@ -377,30 +396,33 @@ __device__ __forceinline__ void sweep_cta(const SweepMaps &maps, const Geom &g, 
 
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     t.i0 = bx * TX;
-    t.j0 = by * BY;
+    t.j0 = by * zc.rows;
     const int L = g.L, M = g.M, N = g.N, XP = g.XP, PS = (int)g.PS;
     t.N = N;
     t.k0 = zc.plane(c);
     t.k1 = zc.plane(c + 1);
-    // rows: cells x = lane, lane + 32 of row w; column warp: one cell per lane, x = 64 of row `lane`
+    // rows: cells x = lane, lane + 32 of row w; column warp: one cell per lane, x = 64 of row `lane`.  A tile
+    // has zc.rows rows, warp zc.rows computes the halo row and the warps between it and the column's idle.
     const bool column = w == 9;
     const int ty = column ? lane : w;
-    t.role = w < 8 ? 0 : (w == 8 ? 1 : 2);
-    t.duty = lane == 0 ? t.role : 0;
+    t.role = column ? 2 : w < zc.rows ? 0 : w == zc.rows ? 1 : 3;
+    t.duty = lane == 0 ? (column ? 2 : w == 8 ? 1 : 0) : 0;
     t.j = t.j0 + ty;
     t.i = t.i0 + (column ? TX : lane);
-    const bool rowok = !column || lane <= BY;
+    const bool rowok = column ? lane <= zc.rows : t.role != 3;
     t.so = rowok ? (ty + 1) * BXW + (column ? TX : lane) + 4 : BXW + 4;
     t.xo = column ? XCOL + lane : ty * TX + lane;  // the column's idle lanes and second cells: cells nobody reads
     t.xd = t.xo + (column ? 1 : TX);
     t.xr = column ? t.xo : lane < 31 ? t.xo + 33 : XCOL + ty;
-    const T rdy = (rowok && t.j < M) ? ax.rdy[t.j] : T(0);
-    t.rdy2 = (dup<T>((rowok && t.j >= 1 && t.j < M) ? ax.rdy2[t.j] : T(0)));
-    t.rdy = (dup<T>(rdy));
-    t.fy = (dup<T>(rdy * s.dtb));
     s.dt *= T(0.25);  // the sweep forms sigma sums of four cells: 0.25 * sum * dt
-    t.lam = (dup<T>(sizeof(T) == 4 ? s.lam2 / s.dt : s.lam2));
-    t.c4 = (dup<T>(sizeof(T) == 4 ? s.c4 / s.dt : s.c4));
+    const T cf = sizeof(T) == 4 ? T(1) : s.c4;  // in the cell sizes of the curl (FP64)
+    t.lam = dup<T>(s.lam2);
+    t.dt = dup<T>(s.dt);
+    t.c4 = dup<T>(sizeof(T) == 4 ? s.c4 : s.lam2 + s.lam2);
+    const T rdy = (rowok && t.j < M) ? ax.rdy[t.j] : T(0);
+    t.rdy2 = dup<T>((rowok && t.j >= 1 && t.j < M) ? ax.rdy2[t.j] * cf : T(0));
+    t.rdy = dup<T>(rdy);
+    t.fy = dup<T>(rdy * s.dtb);
     T r2[2], r1[2];
     t.upd = 0;
 #pragma unroll
@@ -409,7 +431,7 @@ __device__ __forceinline__ void sweep_cta(const SweepMaps &maps, const Geom &g, 
         const int i = t.i + 32 * q;
         const bool ux = act && t.j >= 1 && t.j < M && i < L, uy = act && i >= 1 && i < L && t.j < M;
         t.upd |= (ux ? 1u << q : 0u) | (uy ? 4u << q : 0u);
-        r2[q] = uy ? ax.rdx2[i] : T(0);
+        r2[q] = uy ? ax.rdx2[i] * cf : T(0);
         r1[q] = (act && i < L) ? ax.rdx[i] : T(0);
     }
     t.edge = __any_sync(0xffffffffu, t.upd != 15u);
@@ -423,7 +445,7 @@ __device__ __forceinline__ void sweep_cta(const SweepMaps &maps, const Geom &g, 
         const int k = klow + e;
         const bool in = k >= 0 && k < N;
         s_z[3 * e] = dup<T>(in ? ax.rdz[k] * s.dtb : T(0));
-        s_z[3 * e + 1] = dup<T>(in ? ax.rdzs[k] : T(0));
+        s_z[3 * e + 1] = dup<T>(in ? ax.rdzs[k] * cf : T(0));
         s_z[3 * e + 2] = dup<T>(in ? ax.dzk[k] : T(0));
     }
 
@@ -434,7 +456,7 @@ __device__ __forceinline__ void sweep_cta(const SweepMaps &maps, const Geom &g, 
         if (src.comp[q] == 0) a1 += src.count[q] - 1;
         if (src.comp[q] == 1) b1 += src.count[q] - 1;
         if (src.comp[q] == 2) c1 += src.count[q] - 1;
-        if (a1 >= t.i0 && a0 <= t.i0 + TX && b1 >= t.j0 && b0 <= t.j0 + BY) {
+        if (a1 >= t.i0 && a0 <= t.i0 + TX && b1 >= t.j0 && b0 <= t.j0 + zc.rows) {
             src_tile = true;
             sk0 = min(sk0, src.k[q]);
             sk1 = max(sk1, c1);
@@ -448,12 +470,12 @@ __device__ __forceinline__ void sweep_cta(const SweepMaps &maps, const Geom &g, 
         t.s_src[1] = sk1;
     }
     __syncthreads();
-    if (t.duty == 1) {  // B and sigma of plane ktop through slot 3, stages ktop .. ktop-2 into slots 0..2
-        uint64_t *b = t.bars + 3;
+    if (t.duty == 1) {  // B and sigma of plane ktop through the last slot, the first stages into the others
+        uint64_t *b = t.bars + RING - 1;
         mbar_expect_tx(b, (unsigned)(3 * BOX * sizeof(T)));
         for (int a : {ABX, ABY, ASG})
-            tma_load_3d(t.sm + (3 * NARR + a) * BS, maps.m + a, t.i0, t.j0, ktop + 1, b);
-        for (int q = 0; q < 3 && ktop - q >= t.k0; q++) load_stage(t, ktop - q, q);
+            tma_load_3d(t.sm + ((RING - 1) * NARR + a) * BS, maps.m + a, t.i0, t.j0, ktop + 1, b);
+        for (int q = 0; q < RING - 1 && ktop - q >= t.k0; q++) load_stage(t, ktop - q, q);
     }
     // chunk offsets of Bz over the box (zero without chunking)
     for (int e = tid; e < BOX; e += NT) {
@@ -476,25 +498,27 @@ __device__ __forceinline__ void sweep_cta(const SweepMaps &maps, const Geom &g, 
         s_oc[e] = o;
         s_oc1[e] = o1;
     }
-    t.bad = !mbar_wait_bounded(t.bars + 3, 0u);
+    t.bad = !mbar_wait_bounded(t.bars + RING - 1, 0u);
     if (!t.bad) t.bad = !mbar_wait_bounded(t.bars + 0, 0u);
-    carry_plane(t, t.sm + 3 * NARR * BS);
+    carry_plane<0>(t, t.sm + (RING - 1) * NARR * BS);
     t.ex1 = t.ey1 = t.exn = t.eyn = t.ezn = dup<T>(T(0));
     t.bxo1 = t.byo1 = t.bxn = t.byn = t.acc = dup<T>(T(0));
     async_shared_fence();
     __syncthreads();
-    if (t.duty == 1 && ktop - 3 >= t.k0) load_stage(t, ktop - 3, 3);
+    if (t.duty == 1 && ktop - (RING - 1) >= t.k0) load_stage(t, ktop - (RING - 1), RING - 1);
 
     // Bz offsets of the first plane: ktop is the halo plane k1 of the chunk below (its offsets) or the
     // zero bottom; every later plane lies in this chunk
     set_offsets(t, ktop < N ? s_oc1 : s_oc);
+    t.offsets = c + 1 < zc.n;
     // FP64 (bound by the FP64 pipe): the halo warps run their reduced copies of the plane code
     // (5 % faster).  FP32 runs one copy in every warp: three copies of its loop made the sweep 40 %
     // slower (measured; presumably the larger loop no longer fits the instruction cache).
     if constexpr (sizeof(T) == 8) {
         if (t.role == 0) sweep_march<T, 0>(t, s, s_z, src, s_oc);
         else if (t.role == 1) sweep_march<T, 1>(t, s, s_z, src, s_oc);
-        else sweep_march<T, 2>(t, s, s_z, src, s_oc);
+        else if (t.role == 2) sweep_march<T, 2>(t, s, s_z, src, s_oc);
+        else sweep_march<T, 3>(t, s, s_z, src, s_oc);
     } else {
         sweep_march<T, 0>(t, s, s_z, src, s_oc);
     }
@@ -511,7 +535,7 @@ __device__ __forceinline__ void sweep_cta(const SweepMaps &maps, const Geom &g, 
             atomicExch(err, 1);
             for (int k = t.k0; k <= ktop && k < t.k0 + RING; k++) {
                 const int n = ktop - k;  // stages land in order: slot n % RING, round n / RING
-                mbar_wait_bounded(t.bars + n % RING, (unsigned)(n / RING + (n % RING == 3)) & 1u);
+                mbar_wait_bounded(t.bars + n % RING, (unsigned)(n / RING + (n % RING == RING - 1)) & 1u);
             }
         }
         __syncthreads();

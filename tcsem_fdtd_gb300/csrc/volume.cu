@@ -158,7 +158,7 @@ void launch_fused_sweep(const SweepMaps &maps, const Geom &g, const T *tin, T *t
                         const SourceTable<T> &src, const ZChunks &zc, int c0, int c1, bool rev, int *err,
                         cudaStream_t st, bool pdl) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((g.L + fs3::TX - 1) / fs3::TX, (g.M + fs3::BY - 1) / fs3::BY, c1 - c0);
+    cfg.gridDim = dim3(sweep_tiles_x(g.L), sweep_tiles_y(g.M, zc.rows), c1 - c0);
     cfg.blockDim = dim3(fs3::NT);
     cfg.dynamicSmemBytes = fs3::smem_bytes_n<T>(g.N);
     cfg.stream = st;
@@ -176,7 +176,7 @@ void launch_sweep_batched(const SweepSlot<T> *slots, const BatchIndex &idx, int 
     k_sweep_batched<T><<<idx.total(), fs3::NT, fs3::smem_bytes_n<T>(N_max), st>>>(slots, idx, s, c0);
 }
 int sweep_tiles_x(int L) { return (L + fs3::TX - 1) / fs3::TX; }
-int sweep_tiles_y(int M) { return (M + fs3::BY - 1) / fs3::BY; }
+int sweep_tiles_y(int M, int rows) { return (M + rows - 1) / rows; }
 
 template <typename T> cudaError_t sweep_configure(int N) {
     const int sm = (int)fs3::smem_bytes_n<T>(N);
@@ -194,7 +194,6 @@ template <typename T> int sweep_blocks_per_sm(int N) {
 int sweep_box_x() { return fs3::BXW; }
 int sweep_box_y() { return fs3::BYH; }
 int sweep_tile_x() { return fs3::TX; }
-int sweep_tile_y() { return fs3::BY; }
 
 // materialise Bz = P + O_c in place and clear the chunk totals
 template <typename T>
