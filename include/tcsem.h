@@ -77,7 +77,9 @@ typedef struct {
     size_t device_bytes;  /* device memory held by the handle */
     int launches_per_step; /* kernels launched per time step by tcsem_advance (a batch slot: for
                               all slots together; 0 with persistent_batch, which launches three
-                              kernels per block of graph_steps steps) */
+                              kernels per block of graph_steps steps, and 0 for a small FP32 survey
+                              with the default layout, whose steps run as one cooperative launch
+                              for up to 512 of them) */
     int zchunks;          /* z-chunks of the fused sweep in use */
     int top_planes;       /* planes of the top z-chunk when it runs beside the others, else 0 */
     size_t uploaded_bytes; /* host-to-device bytes the open copied (conductivity, grid, boundary and

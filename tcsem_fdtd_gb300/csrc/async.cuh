@@ -53,6 +53,10 @@ __device__ __forceinline__ int ld_acquire(const int *p) {
 __device__ __forceinline__ void st_release(int *p, int v) {
     asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
+// add with gpu-scope release: what the thread has written or observed is visible to who acquires the sum
+__device__ __forceinline__ void red_release(int *p, int v) {
+    asm volatile("red.release.gpu.global.add.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
 // gpu-scope fence: with a relaxed atomic after it a release, with a relaxed atomic before it an acquire
 __device__ __forceinline__ void fence_acq_rel_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
 // orders this thread's generic-proxy accesses of global memory with its bulk copies (async proxy)

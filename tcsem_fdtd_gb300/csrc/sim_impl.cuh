@@ -32,6 +32,7 @@
 #include "kernels.cuh"
 #include "rx.cuh"
 #include "setup.h"
+#include "steps.cuh"
 #include "tcsem.h"
 
 namespace tcsem {
@@ -200,6 +201,13 @@ template <typename T> struct SimImpl : SimBase {
     int rx_pending = -1;
     StepGate rx_gate{};
     bool overlap = false;
+    // the whole time loop as cooperative launches of many steps (steps.cu)
+    bool steps_on = false;
+    DevMem st_ctl, st_mem;
+    StepsArgs<T> sa{};
+    size_t st_smem = 0;
+    // a launch costs about 8 us (its control words, the resident set-up); between launches other streams get in
+    static constexpr long kStepsPerLaunch = 512;
     bool overlap_pdl = false;  // programmatic dependent launch inside the boundary chain of the overlapped step
 
     ~SimImpl() override {
@@ -287,8 +295,19 @@ template <typename T> struct SimImpl : SimBase {
         dzero(errw.p, sizeof(int));
         init_boundary();
         init_chunks();
+        plan_steps();
+        st_gx = {};
+        st_gy = {};
         init_maps();
         init_steps();
+        if (steps_on) {
+            bind_steps();
+            launches_per_step = 0;
+            chunks_used = zc.n;
+            top_used = zc.n > 1 ? zc.kb[1] : 0;
+            CK(cudaStreamSynchronize(stream));
+            return;
+        }
         // the top chunk's air plane is the only input of the sweep that the boundary writes
         overlap = zc.n > 1 && !opts.serial_boundary;
         if (overlap) {
@@ -456,6 +475,250 @@ template <typename T> struct SimImpl : SimBase {
             CK(cudaMemsetAsync(tot[b].p, 0, tb, stream));
         }
     }
+
+    // ---- cooperative launches of many steps (steps.cu): FP32, the default layout and order
+    std::vector<double> st_gx, st_gy, st_w[4];  // filters [H][M1p] and sampling of the transform lines (init_boundary)
+    std::vector<int> st_i[4];
+    static constexpr int kStepsRx = 2;
+    // Where the cooperative launch is the faster one: where its estimate (steps_layout) is below the graph's, 24 us
+    // or, by the operations of its transforms, more.  It wins by the latency of the graph's boundary chain, four
+    // kernels of 3 to 8 us each; it loses where the sweep leaves so few CTAs that the boundary's phases take
+    // several rounds, and where the sweep keeps the memory busy and every table row a product waits for comes
+    // late.  Measured, us per step with the graph and with the cooperative launch (cells, estimate):
+    // 44 x 38 x 27 (0.05 M, 19) 22.7 and 18.8, 64 x 64 x 48 (0.20 M, 20) 25.8 and 19.2, 160 x 56 x 40 (0.36 M, 24)
+    // 31.9 and 24.3, 79 x 70 x 42 (0.23 M, 19) 25.6 and 16.8, 155 x 67 x 51 (0.53 M, 21) 29.4 and 21.9,
+    // 175 x 60 x 39 (0.41 M, 23) 25.2 and 24.3, 110 x 55 x 153 (0.93 M, 21) 25.7 and 23.0, 135 x 79 x 119 (1.27 M, 41,
+    // a plane of prime length) 84.9 and 39.6; beyond the line 103 x 215 x 35 (0.78 M, 31) 30.5 and 40.5,
+    // 153 x 56 x 144 (1.23 M, 27) 26.3 and 28.5, 253 x 57 x 57 (0.82 M, 31) 29.6 and 34.9, and with more than
+    // 1.3 M cells (chunks freely chosen) 233 x 109 x 65 32.4 and 37.5, 159 x 157 x 125 49.2 and 54.5.
+    static constexpr double kStepsCells = 1.3e6;
+    bool steps_possible() const {
+        return sizeof(T) == 4 && opts.zchunks == 0 && opts.top_planes == 0 && !opts.serial_boundary && !tot_chunks_min &&
+               (double)model.L * model.M * model.N <= kStepsCells;
+    }
+    void plan_steps() {
+        if constexpr (sizeof(T) == 4) {
+            const Model &m = model;
+            if (!steps_possible()) return;
+            const int L1 = bd.L1, M1 = bd.M1;
+            Products<T> &d = sa.pd;
+            products_shape(d, m.L, m.M, L1, M1, true);
+            if (!steps_layout()) return;
+            const Remap Px = remap_lists(m.sl, m.sr, m.ox, m.AnLx_New + m.in.Nx, bd.AL, m.in.Nx, m.AnLx_New, m.L,
+                                         L1, bd.Lu, bd.DL, pad_weights(L1, bd.Lu, bd.DL));
+            const Remap Py = remap_lists(m.sf, m.sb, m.oy, m.Any_New + m.in.Ny, bd.Ay, m.in.Ny, m.Any_New, m.M,
+                                         M1, bd.Mu, bd.DM, pad_weights(M1, bd.Mu, bd.DM));
+            if (!symmetric(Py, m.M, M1, st_i[1], st_w[1], st_i[3], st_w[3])) {
+                products_shape(d, m.L, m.M, L1, M1, false);
+                if (!steps_layout()) return;
+            }
+            init_products(Px, Py);
+            steps_on = true;
+        }
+    }
+    // sweep and boundary CTAs and frequencies per CTA of the cooperative launch; false: the captured graph is faster
+    bool steps_layout() {
+        if constexpr (sizeof(T) == 4) {
+            const Model &m = model;
+            const Products<T> &d = sa.pd;
+            st_smem = steps_smem(d, m.N);
+            int maxsm = 0;
+            CK(cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
+            if (st_smem > (size_t)maxsm) return false;
+            CK(steps_configure<T>(maxsm));  // the most for any grid: the limit is the function's, not the handle's
+            const int slots = steps_blocks<T>(st_smem), tiles = sweep_tiles_x(m.L) * sweep_tiles_y(m.M, zc.rows);
+            sa.nfwd = tiles_fwd(d);
+            sa.ninv = tiles_inv(d);
+            sa.tiles_x = sweep_tiles_x(m.L);
+            sa.tiles = tiles;
+            sa.nrx = kStepsRx;
+            // The fastest estimate (us).  A phase of the boundary takes its blocks in rounds of its CTAs; `march` CTAs
+            // of every tile take the lower chunks in turn, and others or the last of these the top one.  A launch
+            // that leaves room for another one or two (several handles at once) is taken when it costs at most 6 %
+            // more.
+            const double kb = d.K * (2.0 * d.Mh + 8.0 * (up(d.Rx, 4) + up(d.Ry, 4))) * sizeof(T) / 1024;
+            const int lower = zc.n - 1, deep = zc.kb[zc.n] - zc.kb[zc.n - 1];
+            double best = 1e30, least = 1e30;
+            for (int share = 1; share <= 3; share++) {
+                StepsArgs<T> pick = sa;
+                double t_share = 1e30;
+                for (int march = std::max(1, lower); march >= 1; march--)
+                    for (int own = lower > 0; own >= 0; own--)
+                        for (int ncol = 1; ncol <= 2; ncol++) {
+                            const int sweep = (march + own) * tiles, room = slots / share - kStepsRx - sweep,
+                                      through = up(bd.H, ncol);
+                            if (room < 32) continue;
+                            const int w = std::min(room, std::max({sa.nfwd, sa.ninv, through}));
+                            // a second round finds nothing under way; a top chunk behind others starts late
+                            auto rounds = [&](int blocks, double us) { return us + (us + 2.0) * (up(blocks, w) - 1); };
+                            const double fwd = rounds(sa.nfwd, 1.0 + 0.017 * m.L + 0.12 * zc.n),
+                                         thr = rounds(through, ncol == 1 ? 1.8 + 0.015 * kb : 2.0 + 0.03 * kb),
+                                         inv = rounds(sa.ninv, 1.4 + 0.0063 * d.nc),
+                                         calls = up(std::max(1, lower), march),
+                                         low = 2.6 + calls * (3.0 + 0.8 * (deep + 2)) * (calls > 1 ? 1.25 : 1.0),
+                                         shared = sweep + w + kStepsRx > slots / 2 ? 1.3 : 0.0,  // two CTAs on an SM
+                                         t = std::max(fwd + thr + inv + (own ? 8.6 : 9.4), low + (own ? 0.0 : 5.0)) + 1.3 + shared;
+                            if (t < t_share - 1e-9) {
+                                t_share = t;
+                                pick.march = march;
+                                pick.own = own;
+                                pick.nsweep = sweep;
+                                pick.nbnd = w;
+                                pick.ncol = ncol;
+                            }
+                        }
+                least = std::min(least, t_share);
+                if (t_share <= 1.06 * least) best = t_share, sa = pick;
+            }
+            const double work = (((m.M + 1) / 2 + bd.S) * fft_ops(bd.px) + 3.0 * bd.H * fft_ops(bd.py));
+            return best <= std::max(24.0, 20.5 + 0.6e-6 * work);  // the graph's
+        }
+        return false;
+    }
+    // the spline remap of one axis onto the transform line of n points (offset d, nu points on the grid; the points
+    // beyond it taper from the edge values with the weights pad): the weights of each cell at its points
+    struct Remap {
+        std::vector<int> off{0}, lo;
+        std::vector<double> w;
+        double at(int i, int p) const {
+            return p >= lo[i] && p < lo[i] + off[i + 1] - off[i] ? w[off[i] + p - lo[i]] : 0.0;
+        }
+    };
+    static Remap remap_lists(const SplinePlan &a, const SplinePlan &b, int b_src, int b_dst, int lead, int core, int core_dst,
+                             int cells, int n, int nu, int d, const std::vector<double> &pad) {
+        Remap m;
+        std::vector<double> col(n, 0.0), y, mb;
+        auto strip = [&](const SplinePlan &S, int q, int dst) {  // node q of a strip
+            if (q < 0 || q >= S.n) return;
+            y.assign(S.n, 0.0);
+            mb.assign(S.n, 0.0);
+            y[q] = 1.0;
+            for (int i = 1; i < S.n - 1; i++)
+                mb[i] = (y[i + 1] - y[i]) * S.g[i] - (y[i] - y[i - 1]) * S.g[i - 1] - S.w[i] * mb[i - 1];
+            mb[S.n - 1] = 0.0;
+            for (int i = S.n - 2; i >= 1; i--) mb[i] = (mb[i] - S.du[i] * mb[i + 1]) * S.inv[i];
+            mb[0] = 0.0;
+            for (int p = 0; p < S.npts; p++)
+                for (int j = 0; j < 3; j++)
+                    col[d + dst + p] += S.c[(size_t)j * S.npts + p] * y[S.k0[p] + j] +
+                                        S.c[(size_t)(3 + j) * S.npts + p] * mb[S.k0[p] + j];
+        };
+        for (int i = 0; i < cells; i++) {
+            strip(a, i, 0);
+            strip(b, i - b_src, b_dst);
+            if (i >= lead && i < lead + core) col[d + core_dst + i - lead] = 1.0;
+            const double e0 = col[d], e1 = col[d + nu - 1];
+            if (e0 != 0.0)
+                for (int p = 0; p < d; p++) col[p] = pad[p] * e0;
+            if (e1 != 0.0)
+                for (int p = d + nu; p < n; p++) col[p] = pad[p] * e1;
+            int lo = 0, hi = n;
+            while (lo < hi && col[lo] == 0.0) lo++;
+            while (hi > lo && col[hi - 1] == 0.0) hi--;
+            m.lo.push_back(lo);
+            m.w.insert(m.w.end(), col.begin() + lo, col.begin() + hi);
+            m.off.push_back((int)m.w.size());
+            std::fill(col.begin() + lo, col.begin() + hi, 0.0);
+        }
+        return m;
+    }
+    // whether the y line and its sampling are their own mirror images
+    static bool symmetric(const Remap &Py, int M, int M1, const std::vector<int> &xj,
+                          const std::vector<double> &xv, const std::vector<int> &yj, const std::vector<double> &yv) {
+        double worst = 0;
+        for (int p = 0; p < M1; p++)
+            for (int j = 0; j < M; j++)
+                worst = std::max(worst, std::fabs(Py.at(j, p) - Py.at(M - 1 - j, M1 - 1 - p)));
+        auto line = [&](const std::vector<int> &at, const std::vector<double> &w) {
+            const int n = (int)at.size();
+            auto weight = [&](int r, int p) { return p == at[r] ? 1.0 - w[r] : p == at[r] + 1 ? w[r] : 0.0; };
+            for (int r = 0; r < n; r++)
+                for (int p = at[r]; p <= at[r] + 1; p++)
+                    worst = std::max(worst, std::fabs(weight(r, p) - weight(n - 1 - r, M1 - 1 - p)));
+        };
+        line(xj, xv);
+        line(yj, yv);
+        return worst < 1e-9;
+    }
+    void init_products(const Remap &Px, const Remap &Py) {
+        Products<T> &d = sa.pd;
+        size_t n[kProductArrays], at[kProductArrays + 1] = {0};
+        products_sizes(d, n);
+        for (int q = 0; q < kProductArrays; q++) at[q + 1] = at[q] + (size_t)up((int)n[q], 64) * 64;
+        st_mem.alloc(at[kProductArrays] * sizeof(T));
+        dev_bytes += st_mem.n;
+        CK(cudaMemsetAsync(st_mem.p, 0, st_mem.n, stream));
+        T *p[kProductArrays];
+        for (int q = 0; q < kProductArrays; q++) p[q] = st_mem.as<T>() + at[q];
+        products_bind(d, p);
+        d.err = errw.as<int>();
+        // one copy: the remaps, the sampling and (last, in place) the filters of ky = 0 .. M1/2, where a frequency
+        // and its negative share one entry
+        std::vector<unsigned char> h;
+        auto put = [&](const auto &v) {
+            const size_t o = h.size();
+            h.resize(o + (v.size() * sizeof(v[0]) + 15) / 16 * 16);
+            std::memcpy(h.data() + o, v.data(), v.size() * sizeof(v[0]));
+            return o;
+        };
+        const size_t o[6] = {put(Px.off), put(Px.lo), put(Px.w), put(Py.off), put(Py.lo), put(Py.w)};
+        size_t oi[4], ow[4];
+        for (int q = 0; q < 4; q++) {
+            oi[q] = put(st_i[q]);
+            ow[q] = put(st_w[q]);
+        }
+        DevMem t;
+        t.alloc(h.size() + 2 * (size_t)(bd.L1 + bd.M1) * sizeof(double2));
+        unsigned char *b = t.as<unsigned char>();
+        CK(cudaMemcpyAsync(b, h.data(), h.size(), cudaMemcpyHostToDevice, stream));
+        uploaded_bytes += h.size();
+        auto ints = [&](size_t q) { return reinterpret_cast<const int *>(b + q); };
+        auto dbls = [&](size_t q) { return reinterpret_cast<const double *>(b + q); };
+        const LineSampling smp{ints(oi[0]), ints(oi[1]), ints(oi[2]), ints(oi[3]),
+                               dbls(ow[0]), dbls(ow[1]), dbls(ow[2]), dbls(ow[3])};
+        CK(products_tables(d, bd.L1, LineRemap{ints(o[0]), ints(o[1]), dbls(o[2])}, LineRemap{ints(o[3]), ints(o[4]), dbls(o[5])},
+                           smp, reinterpret_cast<double2 *>(b + h.size()), stream));
+        const double norm = 1.0 / ((double)bd.L1 * bd.M1);
+        std::vector<T> f(at[5] - at[3], T(0));
+        for (int a = 0; a < 2; a++)
+            for (int kx = 0; kx < bd.H; kx++)
+                for (int ky = 0; ky <= bd.M1 / 2; ky++)
+                    f[(a ? at[4] - at[3] : 0) + (size_t)kx * d.ldG + ky] =
+                        (T)((a ? st_gy : st_gx)[(size_t)kx * bd.M1p + ky] * (ky == 0 || 2 * ky == bd.M1 ? 1.0 : 2.0) * norm);
+        CK(cudaMemcpyAsync(p[3], f.data(), f.size() * sizeof(T), cudaMemcpyHostToDevice, stream));
+        uploaded_bytes += f.size() * sizeof(T);
+        CK(cudaStreamSynchronize(stream));  // the temporaries are freed on return
+    }
+    void bind_steps() {
+        if constexpr (sizeof(T) == 4) {
+            st_ctl.alloc(kStWords * sizeof(int));
+            dev_bytes += st_ctl.n;
+            for (int b = 0; b < 2; b++) {
+                sa.maps[b] = maps[b];
+                sa.f[b] = fs(b);
+                sa.tot[b] = tot[b].as<T>();
+            }
+            sa.g = g; sa.ax = ax; sa.table = steps.as<StepScalars<T>>(); sa.zc = zc;
+            sa.ctl = st_ctl.as<int>();
+            sa.err = errw.as<int>();
+            sa.wait_ns = 2000000000LL;
+        }
+    }
+    void advance_steps(long todo) {
+        if constexpr (sizeof(T) == 4) {
+            sa.src = src;
+            sa.rd = rd;
+            while (todo > 0) {
+                sa.step0 = step;
+                sa.n = (int)std::min(todo, kStepsPerLaunch);
+                sa.cur = cur;
+                CK(launch_steps<T>(sa, st_smem, stream));
+                step += sa.n;
+                todo -= sa.n;
+                cur ^= sa.n & 1;
+            }
+        }
+    }
     void init_maps() {
         if (g.total() >= (1LL << 31)) throw Error(TCSEM_ERR_INVALID, "grid too large for 32-bit offsets");
         EncodeTiledFn enc = encode_tiled();
@@ -594,8 +857,8 @@ template <typename T> struct SimImpl : SimBase {
         std::vector<double> gx((size_t)H * M1p, 0.0), gy((size_t)H * M1p, 0.0);
         const double dxm = m.in.dxmin, dym = m.in.dymin, dzm = m.in.dzmin;
         for (int kx = 0; kx < H; kx++)
-            for (int ky = 0; ky < M1; ky++) {
-                double v1 = ky < M1 / 2 + 1 ? (1.0 * kPi * ky) / M1 * (dzm / dym) : -(1.0 * kPi * (M1 - ky)) / M1 * (dzm / dym);
+            for (int ky = 0; ky < M1 / 2 + 1; ky++) {  // -ky at M1 - ky: the same a, the opposite b
+                double v1 = (1.0 * kPi * ky) / M1 * (dzm / dym);
                 double u1 = (1.0 * kPi * kx) / L1 * (dzm / dxm);
                 double a, b;
                 if (kx == 0 && ky == 0) { a = 1.0; b = 1.0; }
@@ -607,6 +870,10 @@ template <typename T> struct SimImpl : SimBase {
                 }
                 gx[(size_t)kx * M1p + ky] = a;
                 gy[(size_t)kx * M1p + ky] = b;
+                if (ky > 0 && 2 * ky < M1) {
+                    gx[(size_t)kx * M1p + M1 - ky] = a;
+                    gy[(size_t)kx * M1p + M1 - ky] = -b;
+                }
             }
         for (int kx = 0; kx < H; kx++) {
             if (!(kx == 0 || 2 * kx == L1)) continue;
@@ -655,6 +922,15 @@ template <typename T> struct SimImpl : SimBase {
             double Yp = j == m.M ? m.Y[m.M - 1] + 0.5 * m.dy[m.M - 1] : m.Y[j] - 0.5 * m.dy[j];
             hbyra[j] = slot[J - 1]; hbyrb[j] = slot[J];
             hbyrl[j] = (Yp - m.Yn[J - 1]) / (m.Yn[J] - m.Yn[J - 1]);
+        }
+        if (steps_possible()) {  // first sampled points and rows of the transform lines (plan_steps)
+            st_gx = std::move(gx);
+            st_gy = std::move(gy);
+            for (int v : hbxcII) st_i[0].push_back(v - 1 + DL);
+            for (int v : hbxra) st_i[1].push_back(need[v] + DM);
+            for (int v : hbycII) st_i[2].push_back(v - 1 + DL);
+            for (int v : hbyra) st_i[3].push_back(need[v] + DM);
+            st_w[0] = hbxcl; st_w[1] = hbxrl; st_w[2] = hbycl; st_w[3] = hbyrl;
         }
         upload(bxc_II, hbxcII); upload(bxr_a, hbxra); upload(bxr_b, hbxrb);
         upload(byc_II, hbycII); upload(byr_a, hbyra); upload(byr_b, hbyrb);
@@ -841,6 +1117,10 @@ template <typename T> struct SimImpl : SimBase {
     void advance(long n, int *done) override {
         if (!begun) throw Error(TCSEM_ERR_STATE, "tcsem_begin must precede tcsem_advance");
         long todo = std::min(sched.nsteps - step, std::max(0L, n));
+        if (steps_on) {
+            advance_steps(todo);
+            todo = 0;
+        }
         // whole captured blocks (an even number of steps returns the state to `cur`)
         while (todo >= gsteps) {
             CK(cudaGraphLaunch(graph_for(cur), stream));
@@ -1145,7 +1425,7 @@ template <typename T> struct SimImpl : SimBase {
 
     void timed_advance(long n, double *ms_out) override {
         if (!begun) throw Error(TCSEM_ERR_STATE, "tcsem_begin must precede tcsem_timed_advance");
-        graph_for(cur);  // capture (once) outside the timed region
+        if (!steps_on) graph_for(cur);  // capture (once) outside the timed region
         cudaEvent_t e0, e1;
         CK(cudaEventCreate(&e0));
         CK(cudaEventCreate(&e1));
@@ -1167,8 +1447,10 @@ template <typename T> struct SimImpl : SimBase {
         cudaEvent_t e0, e1;
         CK(cudaEventCreate(&e0));
         CK(cudaEventCreate(&e1));
-        graph_for(cur);  // capture outside the timed region
-        graph_for(cur ^ 1);
+        if (!steps_on) {
+            graph_for(cur);  // capture outside the timed region
+            graph_for(cur ^ 1);
+        }
         CK(cudaStreamSynchronize(stream));
         CK(cudaEventRecord(e0, stream));
         advance(n, nullptr);

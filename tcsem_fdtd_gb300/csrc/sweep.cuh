@@ -153,8 +153,15 @@ template <int ROLE, typename T> __device__ __forceinline__ void carry_plane(Swee
     t.bxj = rcells<ROLE>(p + ABX * BS, so - BXW);
     t.byi = rcells<ROLE>(p + ABY * BS, so - 1);
 }
+// What the loading thread does before it loads the air plane (k = -1), the boundary's output: wait for the
+// previous kernel on the stream (a top chunk launched early, programmatic dependent launch after the
+// boundary's last stage, waits for it there and not before; no-op without the launch attribute).
+struct AirAfterKernel {
+    __device__ __forceinline__ void operator()() const { pdl_wait_prev(); }
+};
 // the loading thread: stage k into slot q
-template <typename T> __device__ __forceinline__ void load_stage(const SweepThread<T> &t, int k, int q) {
+template <typename T, typename Air>
+__device__ __forceinline__ void load_stage(const SweepThread<T> &t, int k, int q, const Air &air) {
     using namespace fs3;
     uint64_t *b = t.bars + q;
     T *dst = t.sm + q * NARR * boxs<T>();
@@ -165,9 +172,7 @@ template <typename T> __device__ __forceinline__ void load_stage(const SweepThre
     box(AEZ, k);
     box(ABZ, k);
     box(ASG, k - 1);
-    // the air plane is the boundary's output: a top chunk launched early (programmatic dependent launch after
-    // the boundary's last stage) waits for it here and not before (no-op without the launch attribute)
-    if (k == 0) pdl_wait_prev();
+    if (k == 0) air();
     box(ABX, k - 1);
     box(ABY, k - 1);
 }
@@ -177,9 +182,9 @@ template <typename T> __device__ __forceinline__ void load_stage(const SweepThre
 // planes' code has no condition on k but the two at the end of the ring.
 enum { FIRST, SECOND, INNER, LAST };
 
-template <typename T, int PH, int KIND, int ROLE>
+template <typename T, int PH, int KIND, int ROLE, typename Air>
 __device__ __forceinline__ void sweep_plane(SweepThread<T> &t, int k, unsigned rp, const StepScalars<T> &s,
-                                            const Pair<T> *zt, const SourceTable<T> &src) {
+                                            const Pair<T> *zt, const SourceTable<T> &src, const Air &air) {
     using namespace fs3;
     typedef Pair<T> P;
     constexpr int BS = boxs<T>(), RING = ring<T>();
@@ -323,7 +328,7 @@ __device__ __forceinline__ void sweep_plane(SweepThread<T> &t, int k, unsigned r
             }
             bulk_commit();
         } else if (KIND != LAST && k - RING >= t.k0) {  // the slot takes the stage RING planes up
-            load_stage(t, k - RING, PH % RING);
+            load_stage(t, k - RING, PH % RING, air);
         }
     }
     // ---- Bz(k+1) = Bz(k+2) + dz (dBx/dx + dBy/dy), for the tile's own rows
@@ -347,40 +352,41 @@ template <typename T> __device__ __forceinline__ void set_offsets(SweepThread<T>
 }
 
 // the z-march of one warp through the chunk, in the copy of the plane code for its role
-template <typename T, int ROLE>
+template <typename T, int ROLE, typename Air>
 __device__ __forceinline__ void sweep_march(SweepThread<T> &t, const StepScalars<T> &s, const Pair<T> *s_z,
-                                            const SourceTable<T> &src, const T *s_oc) {
+                                            const SourceTable<T> &src, const T *s_oc, const Air &air) {
     using namespace fs3;
     const int k0 = t.k0;
-    sweep_plane<T, 0, FIRST, ROLE>(t, t.ktop, 0u, s, s_z, src);
+    sweep_plane<T, 0, FIRST, ROLE>(t, t.ktop, 0u, s, s_z, src, air);
     set_offsets(t, s_oc);
     // the inner planes k = ktop - 2 .. k0 begin in phase 2; rp: parity of the ring round
     int k = t.ktop - 1;
-    sweep_plane<T, 1, SECOND, ROLE>(t, k, 0u, s, s_z, src);
+    sweep_plane<T, 1, SECOND, ROLE>(t, k, 0u, s, s_z, src, air);
     unsigned rp = 0;
     int left = 2;  // phase of the plane after the last inner one
     while (--k >= k0) {
-        sweep_plane<T, 2, INNER, ROLE>(t, k, rp, s, s_z, src);
+        sweep_plane<T, 2, INNER, ROLE>(t, k, rp, s, s_z, src, air);
         if (--k < k0) { left = 3; break; }
-        sweep_plane<T, 3, INNER, ROLE>(t, k, rp, s, s_z, src);
+        sweep_plane<T, 3, INNER, ROLE>(t, k, rp, s, s_z, src, air);
         rp ^= 1u;
         if (--k < k0) { left = 0; break; }
-        sweep_plane<T, 0, INNER, ROLE>(t, k, rp, s, s_z, src);
+        sweep_plane<T, 0, INNER, ROLE>(t, k, rp, s, s_z, src, air);
         if (--k < k0) { left = 1; break; }
-        sweep_plane<T, 1, INNER, ROLE>(t, k, rp, s, s_z, src);
+        sweep_plane<T, 1, INNER, ROLE>(t, k, rp, s, s_z, src, air);
     }
-    if (left == 0) sweep_plane<T, 0, LAST, ROLE>(t, k, rp, s, s_z, src);
-    else if (left == 1) sweep_plane<T, 1, LAST, ROLE>(t, k, rp, s, s_z, src);
-    else if (left == 2) sweep_plane<T, 2, LAST, ROLE>(t, k, rp, s, s_z, src);
-    else sweep_plane<T, 3, LAST, ROLE>(t, k, rp, s, s_z, src);
+    if (left == 0) sweep_plane<T, 0, LAST, ROLE>(t, k, rp, s, s_z, src, air);
+    else if (left == 1) sweep_plane<T, 1, LAST, ROLE>(t, k, rp, s, s_z, src, air);
+    else if (left == 2) sweep_plane<T, 2, LAST, ROLE>(t, k, rp, s, s_z, src, air);
+    else sweep_plane<T, 3, LAST, ROLE>(t, k, rp, s, s_z, src, air);
 }
 
 // one CTA of the sweep: tile (bx, by) of z-chunk c with the step scalars s.  FRESH: the chunk
 // totals tin may have been written by another CTA of the same launch (persistent schedule).
-template <typename T, bool FRESH = false>
+template <typename T, bool FRESH = false, typename Air = AirAfterKernel>
 __device__ __forceinline__ void sweep_cta(const SweepMaps &maps, const Geom &g, const T *__restrict__ tin,
                                           T *__restrict__ tout, const Axis<T> &ax, StepScalars<T> s,
-                                          const SourceTable<T> &src, const ZChunks &zc, int bx, int by, int c, int *err) {
+                                          const SourceTable<T> &src, const ZChunks &zc, int bx, int by, int c, int *err,
+                                          const Air &air = Air()) {
     using namespace fs3;
     constexpr int BS = boxs<T>(), RING = ring<T>();
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -475,7 +481,7 @@ __device__ __forceinline__ void sweep_cta(const SweepMaps &maps, const Geom &g, 
         mbar_expect_tx(b, (unsigned)(3 * BOX * sizeof(T)));
         for (int a : {ABX, ABY, ASG})
             tma_load_3d(t.sm + ((RING - 1) * NARR + a) * BS, maps.m + a, t.i0, t.j0, ktop + 1, b);
-        for (int q = 0; q < RING - 1 && ktop - q >= t.k0; q++) load_stage(t, ktop - q, q);
+        for (int q = 0; q < RING - 1 && ktop - q >= t.k0; q++) load_stage(t, ktop - q, q, air);
     }
     // chunk offsets of Bz over the box (zero without chunking)
     for (int e = tid; e < BOX; e += NT) {
@@ -505,7 +511,7 @@ __device__ __forceinline__ void sweep_cta(const SweepMaps &maps, const Geom &g, 
     t.bxo1 = t.byo1 = t.bxn = t.byn = t.acc = dup<T>(T(0));
     async_shared_fence();
     __syncthreads();
-    if (t.duty == 1 && ktop - (RING - 1) >= t.k0) load_stage(t, ktop - (RING - 1), RING - 1);
+    if (t.duty == 1 && ktop - (RING - 1) >= t.k0) load_stage(t, ktop - (RING - 1), RING - 1, air);
 
     // Bz offsets of the first plane: ktop is the halo plane k1 of the chunk below (its offsets) or the
     // zero bottom; every later plane lies in this chunk
@@ -515,12 +521,12 @@ __device__ __forceinline__ void sweep_cta(const SweepMaps &maps, const Geom &g, 
     // (5 % faster).  FP32 runs one copy in every warp: three copies of its loop made the sweep 40 %
     // slower (measured; presumably the larger loop no longer fits the instruction cache).
     if constexpr (sizeof(T) == 8) {
-        if (t.role == 0) sweep_march<T, 0>(t, s, s_z, src, s_oc);
-        else if (t.role == 1) sweep_march<T, 1>(t, s, s_z, src, s_oc);
-        else if (t.role == 2) sweep_march<T, 2>(t, s, s_z, src, s_oc);
-        else sweep_march<T, 3>(t, s, s_z, src, s_oc);
+        if (t.role == 0) sweep_march<T, 0>(t, s, s_z, src, s_oc, air);
+        else if (t.role == 1) sweep_march<T, 1>(t, s, s_z, src, s_oc, air);
+        else if (t.role == 2) sweep_march<T, 2>(t, s, s_z, src, s_oc, air);
+        else sweep_march<T, 3>(t, s, s_z, src, s_oc, air);
     } else {
-        sweep_march<T, 0>(t, s, s_z, src, s_oc);
+        sweep_march<T, 0>(t, s, s_z, src, s_oc, air);
     }
     // the last plane's Bz, in the buffer of its parity
     async_shared_fence();
