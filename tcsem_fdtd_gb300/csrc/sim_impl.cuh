@@ -174,6 +174,8 @@ struct SimBase {
 template <typename T> struct SimImpl : SimBase {
     Geom g{};
     DevMem fld[2][6], con, tot[2];  // two field sets + conductivity; per-set chunk totals of Bz
+    // the current set's totals may be other than zero; shared: others step the sets too (a batch)
+    bool partial = true, shared = false;
     ZChunks zc{0, 8, {}};
     SweepMaps maps[2];              // TMA descriptors of the sweep that reads each field set
     DevMem errw;                    // device error word (a bounded wait gave up)
@@ -758,6 +760,7 @@ template <typename T> struct SimImpl : SimBase {
     void sweep(int b, StepScalars<T> s, const StepScalars<T> *table, StepGate gate, int c0 = 0, int c1 = -1,
                cudaStream_t st = nullptr, bool pdl = false) {
         if (c1 < 0) c1 = zc.n;
+        partial = true;
         // Block order: consecutive steps alternate the chunk order (a step starts on the planes
         // the previous one wrote last), except in a launch that includes a top chunk shorter than
         // the others -- its blocks go last, so its short CTAs take the slots the single wave of
@@ -767,7 +770,12 @@ template <typename T> struct SimImpl : SimBase {
         launch_fused_sweep<T>(maps[b], g, tot[b].as<T>(), tot[b ^ 1].as<T>(), ax, s, table, gate, src, zc,
                               c0, c1, short_top || (b & 1) != 0, errw.as<int>(), st ? st : stream, pdl);
     }
-    void consolidate(int b) { launch_bz_consolidate<T>(g, fs(b).bz, tot[b].as<T>(), zc, stream); }
+    // Bz of the current set without chunk offsets; nothing to do between stage calls (it was half of a call's time)
+    void consolidate() {
+        if (!partial) return;
+        launch_bz_consolidate<T>(g, fs(cur).bz, tot[cur].as<T>(), zc, stream);
+        partial = shared;
+    }
 
     // transform length of a uniform line of n points: n itself (mode 0), the power of two
     // above it (mode 1, the LNx2/LMy2 sizes of ModelingSetup.cpp:194-195), or the smallest
@@ -1047,6 +1055,7 @@ template <typename T> struct SimImpl : SimBase {
         for (int b = 0; b < 2; b++) CK(cudaMemsetAsync(tot[b].p, 0, tot[b].n, stream));
         cur = 0;
         step = 0;
+        partial = shared;
     }
 
     void begin(int t) override {
@@ -1117,6 +1126,7 @@ template <typename T> struct SimImpl : SimBase {
     void advance(long n, int *done) override {
         if (!begun) throw Error(TCSEM_ERR_STATE, "tcsem_begin must precede tcsem_advance");
         long todo = std::min(sched.nsteps - step, std::max(0L, n));
+        if (todo > 0) partial = true;
         if (steps_on) {
             advance_steps(todo);
             todo = 0;
@@ -1153,6 +1163,7 @@ template <typename T> struct SimImpl : SimBase {
 
     // ---- batches: the descriptors of one step that reads field set b and writes b ^ 1
     void batch_slot(int b, const int *counter, SweepSlot<T> &sw, BoundarySlot<T> &bs, RxSlot<T> &rs) {
+        partial = shared = true;
         FieldSet<T> in = fs(b), out = fs(b ^ 1);
         sw.maps = maps[b]; sw.g = g; sw.tin = tot[b].as<T>(); sw.tout = tot[b ^ 1].as<T>();
         sw.ax = ax; sw.table = steps.as<StepScalars<T>>(); sw.step_base = counter; sw.nsteps = sched.nsteps;
@@ -1214,12 +1225,12 @@ template <typename T> struct SimImpl : SimBase {
     void need_tx() { if (itx < 0) select(0); }
     void electric_field(double lam, double dt, double wave) override {
         need_tx();
-        consolidate(cur);
+        consolidate();
         launch_update_e<T>(g, fs(cur), con.as<T>(), ax, scal(lam, dt, 0, wave), src, errw.as<int>(), stream);
         CK(cudaGetLastError());
     }
     void bderivate(double dtb) override {
-        consolidate(cur);
+        consolidate();
         launch_bderivate<T>(g, fs(cur), ax, (T)dtb, errw.as<int>(), stream);
         CK(cudaGetLastError());
     }
@@ -1240,7 +1251,6 @@ template <typename T> struct SimImpl : SimBase {
         if (efield) a.e_slot = slot; else a.b_slot = slot;
         launch_rx<T>(rd, fs(cur), tot[cur].as<T>(), zc, g, StepGate{nullptr, 0, 0}, a, stream);
         CK(cudaGetLastError());
-        CK(cudaStreamSynchronize(stream));
         size_t n = (size_t)model.NComp * rd.nr;
         std::vector<T> h(n);
         d2h(h.data(), ef0.as<T>() + (size_t)slot * n, n * sizeof(T));
@@ -1257,7 +1267,7 @@ template <typename T> struct SimImpl : SimBase {
     void get_field(int comp, double *h) override {
         int nx, ny, nz, z0;
         extents(comp, nx, ny, nz, z0);
-        if (comp == TCSEM_BZ) consolidate(cur);
+        if (comp == TCSEM_BZ) consolidate();
         CK(cudaStreamSynchronize(stream));
         DevMem &dm = field_mem(comp, cur);
         std::vector<T> buf((size_t)g.total());
@@ -1398,6 +1408,7 @@ template <typename T> struct SimImpl : SimBase {
             throw;
         }
         if (h.ef0_bytes != (long long)ef0.n || h.efs_bytes != (long long)efs.n) fail(TCSEM_ERR_INVALID, other);
+        partial = true;
         auto get = [&](void *dev, size_t n) {
             buf.resize(n);
             ok = ok && std::fread(buf.data(), 1, n, f) == n;
