@@ -123,6 +123,9 @@ int sweep_box_x();
 int sweep_box_y();
 int sweep_tile_x();
 template <typename T> void launch_bz_consolidate(const Geom &g, T *bz, T *tot, const ZChunks &zc, cudaStream_t st);
+// nx x ny cells of planes k .. k+n-1 of a volume as dense doubles, and back
+template <typename T> void launch_crop(const Geom &g, const T *v, double *out, int nx, int ny, int k, int n, cudaStream_t st);
+template <typename T> void launch_place(const Geom &g, const double *in, T *v, int nx, int ny, int k, int n, cudaStream_t st);
 
 // ------------------------------------------------------------------ batches
 // Several simulations advanced by one launch per kernel: block b of a batched

@@ -1,6 +1,7 @@
-"""The stage calls where their kernels can go wrong: one plane more and fewer than the planes a block of the Bz sum
-holds, cut tiles, and stage calls between fused steps (Bz then carries the totals of its chunks).  The oracle's
-stages with the tolerances of the stage tests (FP64 1e-10, FP32 2e-5 of the largest value)."""
+"""The stage calls and the exchange of fields with the host where their kernels can go wrong: one plane more and
+fewer than the planes a block of the Bz sum holds, cut tiles, volumes of several pieces of the exchange buffer, and
+stage calls between fused steps (Bz then carries the totals of its chunks).  The oracle's stages with the tolerances
+of the stage tests (FP64 1e-10, FP32 2e-5 of the largest value); values that both types hold come back unchanged."""
 import numpy as np
 import pytest
 
@@ -78,3 +79,19 @@ def test_stage_calls_between_fused_steps(case_dir):
             got.append([first] + [sim.get(n) for n in FIELDS])
     for a, b in zip(*got):
         assert rel(a, b) < 1e-10
+
+
+@pytest.mark.parametrize("precision", [64, 32])
+def test_fields_come_back_as_they_were_set(case_dir, precision):
+    """Whole volumes in two pieces of the exchange buffer (24 planes of 290 x 310), and no other field touched."""
+    from tcsem_fdtd_gb300 import Simulation, build
+
+    build.build()
+    d = grid(case_dir, 290, 310, 30)
+    with Simulation(d, precision=precision) as sim:
+        rng = np.random.default_rng(3)
+        want = {n: rng.standard_normal(sim.field_shape(n)).astype(np.float32).astype(np.float64) for n in FIELDS}
+        for n in FIELDS:
+            sim.set(n, want[n])
+        for n in FIELDS:
+            np.testing.assert_array_equal(sim.get(n), want[n])
