@@ -118,15 +118,20 @@ template <typename T> __host__ __device__ inline ColsLayout cols_layout(const Bo
     size_t o = 0;
     l.bar = o; o += 16;
     l.tw = o; o += rnd16(bd.M1 * sizeof(C2<T>));
-    l.tab = o; o += rnd16(bd.ry.nT * sizeof(T));
-    l.tabi = o; o += rnd16(bd.ry.nI * sizeof(int));
-    l.col = o; o += rnd16(bd.M * sizeof(C2<T>));
     l.gx = o; o += rnd16(bd.M1 * sizeof(T));
     l.gy = o; o += rnd16(bd.M1 * sizeof(T));
     l.a = o; o += rnd16(2 * (size_t)bd.M1 * sizeof(C2<T>));
     l.b = o; o += rnd16(2 * (size_t)bd.M1 * sizeof(C2<T>));
-    l.mb = o; o += rnd16(4 * (size_t)bd.ry.nmax * sizeof(T));
-    l.total = o;
+    // The remap's tables, its column and its spline moments lie where the transforms come later: behind the M1
+    // points that the remap writes.  A column of a 736-point plane needs 35 KB instead of 55, so three blocks
+    // instead of two run beside a sweep CTA (256 x 256 x 160, whose step waits for them: 132.4 -> 129.4 us with the
+    // packed sums of fft.cuh; FP64, the boundary alone: 170 -> 160 us).
+    size_t p = l.a + rnd16(bd.M1 * sizeof(C2<T>));
+    l.tab = p; p += rnd16(bd.ry.nT * sizeof(T));
+    l.tabi = p; p += rnd16(bd.ry.nI * sizeof(int));
+    l.col = p; p += rnd16(bd.M * sizeof(C2<T>));
+    l.mb = p; p += rnd16(4 * (size_t)bd.ry.nmax * sizeof(T));
+    l.total = o > p ? o : p;
     return l;
 }
 template <typename T> __host__ __device__ inline RowsInvLayout rows_inv_layout(const BoundaryDev<T> &bd) {

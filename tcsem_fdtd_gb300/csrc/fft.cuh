@@ -24,6 +24,15 @@ namespace fft {
 
 template <typename T> __device__ __forceinline__ C2<T> add(C2<T> a, C2<T> b) { return {a.x + b.x, a.y + b.y}; }
 template <typename T> __device__ __forceinline__ C2<T> sub(C2<T> a, C2<T> b) { return {a.x - b.x, a.y - b.y}; }
+// in FP32 one packed instruction each (128 x 128 x 96, 250 x 250 plane: 36.4 -> 36.0 us per step)
+__device__ __forceinline__ C2<float> add(C2<float> a, C2<float> b) {
+    const float2 r = __fadd2_rn(make_float2(a.x, a.y), make_float2(b.x, b.y));
+    return {r.x, r.y};
+}
+__device__ __forceinline__ C2<float> sub(C2<float> a, C2<float> b) {
+    const float2 r = __ffma2_rn(make_float2(b.x, b.y), make_float2(-1.f, -1.f), make_float2(a.x, a.y));
+    return {r.x, r.y};
+}
 template <typename T> __device__ __forceinline__ C2<T> scale(C2<T> a, T s) { return {a.x * s, a.y * s}; }
 // multiply by -i (forward) or +i (inverse)
 template <bool INV, typename T> __device__ __forceinline__ C2<T> rot(C2<T> a) {
