@@ -10,7 +10,8 @@
 // kernels and then the sweep of every slot's top z-chunk (the only chunk that
 // reads the air plane), on the main stream the sweep of all lower chunks;
 // both join before the receiver kernel.  Each of these is one launch over all
-// slots.  One advance of all step counters ends the block.  A slot whose
+// slots.  Slots of one chunk each (the default) are swept in two pieces or as two groups instead
+// (plan_step).  One advance of all step counters ends the block.  A slot whose
 // run has ended is gated off inside the kernels; slots join (tcsem_batch_add)
 // and leave (tcsem_batch_remove) between graph launches, which rebuilds the
 // tables and re-captures the graph.  Admission is by device memory: a slot is
@@ -53,12 +54,22 @@ template <typename T> struct BatchImpl : BatchBase {
     size_t used = 0;
     cudaStream_t stream = nullptr;
     DevMem counters, dsw[2], dbs[2], drs[2];
-    BatchIndex itop{}, ilow{}, irs{}, ibs[4]{};  // sweep: chunk 0 of every slot, chunks 1.. of every slot
+    // The blocks of consecutive rows [r0, r1) of the tables; sweep: chunk 0 of every slot, chunks 1.. of every slot
+    struct Group {
+        int r0 = 0, r1 = 0;
+        BatchIndex itop{}, ilow{}, irs{}, ibs[4]{};
+        cudaStream_t stream = nullptr;  // groups after the first
+        cudaEvent_t ev = nullptr;
+    };
+    static constexpr int kGroups = 2;
+    Group groups[kGroups];
+    int ngroups = 1;
+    bool pieces = false, spread = false;
     cudaStream_t side = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     size_t smem_bnd[3] = {0, 0, 0};
     int nmax = 0;
-    int lps = 6;  // launches per step for all slots (a seventh when some slot has lower z-chunks)
+    int lps = 6;  // launches per step for all slots (a seventh when some slot has lower z-chunks; see plan_step)
     cudaGraphExec_t gexec = nullptr;
     int gsteps = 64;
     bool dirty = true;
@@ -82,6 +93,10 @@ template <typename T> struct BatchImpl : BatchBase {
         slots.clear();
         if (ev_fork) cudaEventDestroy(ev_fork);
         if (ev_join) cudaEventDestroy(ev_join);
+        for (Group &g : groups) {
+            if (g.ev) cudaEventDestroy(g.ev);
+            if (g.stream) cudaStreamDestroy(g.stream);
+        }
         if (side) cudaStreamDestroy(side);
         if (stream) cudaStreamDestroy(stream);
     }
@@ -151,6 +166,47 @@ template <typename T> struct BatchImpl : BatchBase {
         return slots.back().id;
     }
 
+    // How a step's boundary runs beside its sweep when every slot is swept in one chunk, whose march reads the air
+    // plane only at its top plane (all of them give the same bits):
+    //  * pieces: the boundary beside the sweep of all but the top planes, then these (7 launches per step).  While
+    //    few tiles leave whole SMs free, one sweep CTA per SM (spread): two on one march half as fast.
+    //  * groups: two halves of the slots on streams of their own, the boundary of one beside the sweep of the other,
+    //    where the tiles of all slots leave the boundary no room.
+    // us per step as one launch after the other, in pieces, spread too, and in two groups (FP32, tiles):
+    // 2 surveys of 44 x 38 x 27 (10) 45, 35, 34, 45; 8 of up to 64 x 64 x 48 (52) 65, 70, 57, 67; 2 of 128 x 128 x 96 (62)
+    // 110, 116, 95, 108; 6 of 95 x 67 x 39 (90) 69, 59, 53, 72; 6 of 119 x 83 x 43 (114) 95, 75, 94, 91; 4 of
+    // 145 x 117 x 61 (150) 115, 93, 93, 109; 8 of 152 x 131 x 112 (300) 196, 195, -, 175; 4 of 200 x 180 x 120 (330) 206, 202,
+    // -, 185.
+    void plan_step() {
+        const int n = (int)running.size();
+        bool whole = !persistent && n > 0;
+        long tiles = 0;
+        for (int q : running) {
+            const SimImpl<T> &m = *slots[q].sim;
+            whole = whole && m.zc.n == 1 && m.g.N >= 2;
+            tiles += m.sweep_blocks();
+        }
+        int sms = 0;
+        CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+        const long slots_sm = sizeof(T) == 4 ? 2 : 1;
+        pieces = whole && 10 * tiles <= 7 * slots_sm * sms;
+        spread = pieces && 3 * tiles <= 2 * sms;
+        ngroups = whole && !pieces && n > 1 ? 2 : 1;
+        std::vector<int> order;  // the running slots dealt out to the groups one by one
+        for (int q = 0, r = 0; q < ngroups; q++) {
+            Group &gr = groups[q];
+            gr.r0 = r;
+            for (int i = q; i < n; i += ngroups, r++) order.push_back(running[i]);
+            gr.r1 = r;
+            gr.itop = BatchIndex{}; gr.ilow = BatchIndex{}; gr.irs = BatchIndex{};
+            gr.itop.n = gr.ilow.n = gr.irs.n = r - gr.r0;
+            for (auto &b : gr.ibs) b = BatchIndex{}, b.n = r - gr.r0;
+            if (q && !gr.stream) CK(cudaStreamCreateWithFlags(&gr.stream, cudaStreamNonBlocking));
+            if (q && !gr.ev) CK(cudaEventCreateWithFlags(&gr.ev, cudaEventDisableTiming));
+        }
+        running = order;
+    }
+
     // tables, block lists and graph for the slots still running
     void rebuild() {
         CK(cudaStreamSynchronize(stream));  // the tables are read by launches in flight
@@ -172,10 +228,7 @@ template <typename T> struct BatchImpl : BatchBase {
         std::vector<BoundarySlot<T>> hbs[2];
         std::vector<RxSlot<T>> hrs[2];
         std::vector<int> hc(kMaxSlots, 0);
-        itop = BatchIndex{}; ilow = BatchIndex{}; irs = BatchIndex{};
-        for (auto &b : ibs) b = BatchIndex{};
-        itop.n = ilow.n = irs.n = n;
-        for (auto &b : ibs) b.n = n;
+        plan_step();
         smem_bnd[0] = smem_bnd[1] = smem_bnd[2] = 0;
         nmax = 0;
         int *cnt = counters.as<int>();
@@ -190,13 +243,16 @@ template <typename T> struct BatchImpl : BatchBase {
             hc[r] = (int)s.done;
             const BoundaryBlocks bb = boundary_blocks(m.bd, m.g);
             const int per_chunk = m.sweep_blocks() / m.zc.n;
-            itop.off[r + 1] = itop.off[r] + per_chunk;
-            ilow.off[r + 1] = ilow.off[r] + per_chunk * (m.zc.n - 1);
-            ibs[0].off[r + 1] = ibs[0].off[r] + bb.rows_fwd;
-            ibs[1].off[r + 1] = ibs[1].off[r] + bb.cols;
-            ibs[2].off[r + 1] = ibs[2].off[r] + bb.rows_inv;
-            ibs[3].off[r + 1] = ibs[3].off[r] + bb.bilinear;
-            irs.off[r + 1] = irs.off[r] + rx_blocks(m.rx_stencils());
+            Group *gr = groups;
+            while (r >= gr->r1) gr++;
+            const int o = r - gr->r0;
+            gr->itop.off[o + 1] = gr->itop.off[o] + per_chunk;
+            gr->ilow.off[o + 1] = gr->ilow.off[o] + per_chunk * (m.zc.n - 1);
+            gr->ibs[0].off[o + 1] = gr->ibs[0].off[o] + bb.rows_fwd;
+            gr->ibs[1].off[o + 1] = gr->ibs[1].off[o] + bb.cols;
+            gr->ibs[2].off[o + 1] = gr->ibs[2].off[o] + bb.rows_inv;
+            gr->ibs[3].off[o + 1] = gr->ibs[3].off[o] + bb.bilinear;
+            gr->irs.off[o + 1] = gr->irs.off[o] + rx_blocks(m.rx_stencils());
             const int it[kStages] = {bb.rows_fwd, bb.cols, bb.rows_inv, (m.g.L + 1) * m.g.M + m.g.L * (m.g.M + 1),
                                      m.sweep_blocks(), m.rx_stencils()};
             for (int q = 0; q < kStages; q++) pa.nitems[r][q] = it[q];
@@ -214,7 +270,7 @@ template <typename T> struct BatchImpl : BatchBase {
         CK(cudaMemcpyAsync(counters.p, hc.data(), kMaxSlots * sizeof(int), cudaMemcpyHostToDevice, stream));
         CK(cudaStreamSynchronize(stream));
         dirty = false;
-        lps = 6 + (ilow.total() > 0 ? 1 : 0);
+        lps = 6 * ngroups + (pieces || groups[0].ilow.total() > 0 ? 1 : 0);
         if (!n) return;
         CK(sweep_configure<T>(nmax));
         CK(boundary_configure_batched<T>(smem_bnd));
@@ -261,16 +317,46 @@ template <typename T> struct BatchImpl : BatchBase {
         // steps alternate the field sets: every slot starts a block in set 0 (blocks have an even length)
         cudaGraph_t graph;
         CK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-        for (int s = 0; s < gsteps; s++) {
+        if (ngroups > 1) {  // each group's steps on a stream of its own
+            CK(cudaEventRecord(ev_fork, stream));
+            for (int q = 0; q < ngroups; q++) {
+                const Group &gr = groups[q];
+                cudaStream_t st = q ? gr.stream : stream;
+                if (q) CK(cudaStreamWaitEvent(st, ev_fork, 0));
+                for (int s = 0; s < gsteps; s++) {
+                    const int p = s & 1;
+                    launch_boundary_batched<T>(dbs[p].as<BoundarySlot<T>>() + gr.r0, gr.ibs, smem_bnd, s, st);
+                    launch_sweep_batched<T>(dsw[p].as<SweepSlot<T>>() + gr.r0, gr.itop, s, 0, nmax, st);
+                    launch_rx_batched<T>(drs[p].as<RxSlot<T>>() + gr.r0, gr.irs, s, st);
+                }
+                if (q) {
+                    CK(cudaEventRecord(gr.ev, st));
+                    CK(cudaStreamWaitEvent(stream, gr.ev, 0));
+                }
+            }
+        }
+        const Group &g0 = groups[0];
+        for (int s = 0; s < gsteps && pieces; s++) {
             const int p = s & 1;
             CK(cudaEventRecord(ev_fork, stream));
             CK(cudaStreamWaitEvent(side, ev_fork, 0));
-            launch_boundary_batched<T>(dbs[p].as<BoundarySlot<T>>(), ibs, smem_bnd, s, side);
-            launch_sweep_batched<T>(dsw[p].as<SweepSlot<T>>(), itop, s, 0, nmax, side);
-            launch_sweep_batched<T>(dsw[p].as<SweepSlot<T>>(), ilow, s, 1, nmax, stream);
+            launch_boundary_batched<T>(dbs[p].as<BoundarySlot<T>>(), g0.ibs, smem_bnd, s, side);
+            launch_sweep_batched<T>(dsw[p].as<SweepSlot<T>>(), g0.itop, s, 0, nmax, stream, Piece::LOWER, spread);
             CK(cudaEventRecord(ev_join, side));
             CK(cudaStreamWaitEvent(stream, ev_join, 0));
-            launch_rx_batched<T>(drs[p].as<RxSlot<T>>(), irs, s, stream);
+            launch_sweep_batched<T>(dsw[p].as<SweepSlot<T>>(), g0.itop, s, 0, nmax, stream, Piece::TOP);
+            launch_rx_batched<T>(drs[p].as<RxSlot<T>>(), g0.irs, s, stream);
+        }
+        for (int s = 0; s < gsteps && ngroups == 1 && !pieces; s++) {
+            const int p = s & 1;
+            CK(cudaEventRecord(ev_fork, stream));
+            CK(cudaStreamWaitEvent(side, ev_fork, 0));
+            launch_boundary_batched<T>(dbs[p].as<BoundarySlot<T>>(), g0.ibs, smem_bnd, s, side);
+            launch_sweep_batched<T>(dsw[p].as<SweepSlot<T>>(), g0.itop, s, 0, nmax, side);
+            launch_sweep_batched<T>(dsw[p].as<SweepSlot<T>>(), g0.ilow, s, 1, nmax, stream);
+            CK(cudaEventRecord(ev_join, side));
+            CK(cudaStreamWaitEvent(stream, ev_join, 0));
+            launch_rx_batched<T>(drs[p].as<RxSlot<T>>(), g0.irs, s, stream);
         }
         launch_advance_all(counters.as<int>(), n, gsteps, stream);
         cudaError_t e = cudaStreamEndCapture(stream, &graph);

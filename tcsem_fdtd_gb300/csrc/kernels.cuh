@@ -147,11 +147,16 @@ struct BatchIndex {
 };
 
 // everything one step of the fused sweep needs for one slot (device memory)
+// A launch may take a chunk in two: all but its top plane, and after that the top plane, whose Bz goes on from the
+// plane below it (the same sums in the same order as the whole chunk's)
+enum class Piece { WHOLE, LOWER, TOP };
+
 template <typename T> struct SweepSlot {
     SweepMaps maps;
     Geom g;
     const T *tin;
     T *tout;
+    const T *bz_new;  // the Bz volume the sweep writes (Piece::TOP)
     Axis<T> ax;
     const StepScalars<T> *table;  // per step of the slot's run
     const int *step_base;         // the slot's step counter; step = *step_base + s
@@ -163,7 +168,8 @@ template <typename T> struct SweepSlot {
 };
 // the blocks of each slot cover its chunks c0, c0+1, ... (tiles_x * tiles_y blocks per chunk)
 template <typename T>
-void launch_sweep_batched(const SweepSlot<T> *slots, const BatchIndex &idx, int s, int c0, int N_max, cudaStream_t st);
+void launch_sweep_batched(const SweepSlot<T> *slots, const BatchIndex &idx, int s, int c0, int N_max, cudaStream_t st,
+                          Piece piece = Piece::WHOLE, bool spread = false);
 int sweep_tiles_x(int L);
 int sweep_tiles_y(int M, int rows);
 

@@ -1167,7 +1167,7 @@ template <typename T> struct SimImpl : SimBase {
     void batch_slot(int b, const int *counter, SweepSlot<T> &sw, BoundarySlot<T> &bs, RxSlot<T> &rs) {
         partial = shared = true;
         FieldSet<T> in = fs(b), out = fs(b ^ 1);
-        sw.maps = maps[b]; sw.g = g; sw.tin = tot[b].as<T>(); sw.tout = tot[b ^ 1].as<T>();
+        sw.maps = maps[b]; sw.g = g; sw.tin = tot[b].as<T>(); sw.tout = tot[b ^ 1].as<T>(); sw.bz_new = out.bz;
         sw.ax = ax; sw.table = steps.as<StepScalars<T>>(); sw.step_base = counter; sw.nsteps = sched.nsteps;
         sw.src = src; sw.zc = zc; sw.err = errw.as<int>();
         sw.tiles_x = sweep_tiles_x(g.L); sw.tiles_y = sweep_tiles_y(g.M, zc.rows);

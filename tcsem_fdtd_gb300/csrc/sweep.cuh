@@ -380,13 +380,14 @@ __device__ __forceinline__ void sweep_march(SweepThread<T> &t, const StepScalars
     else sweep_plane<T, 3, LAST, ROLE>(t, k, rp, s, s_z, src, air);
 }
 
-// one CTA of the sweep: tile (bx, by) of z-chunk c with the step scalars s.  FRESH: the chunk
+// one CTA of the sweep: tile (bx, by) of z-chunk c (or a piece of the only chunk) with the step scalars s.  FRESH: the chunk
 // totals tin may have been written by another CTA of the same launch (persistent schedule).
 template <typename T, bool FRESH = false, typename Air = AirAfterKernel>
 __device__ __forceinline__ void sweep_cta(const SweepMaps &maps, const Geom &g, const T *__restrict__ tin,
                                           T *__restrict__ tout, const Axis<T> &ax, StepScalars<T> s,
                                           const SourceTable<T> &src, const ZChunks &zc, int bx, int by, int c, int *err,
-                                          const Air &air = Air()) {
+                                          const Air &air = Air(), Piece piece = Piece::WHOLE,
+                                          const T *__restrict__ bz_new = nullptr) {
     using namespace fs3;
     constexpr int BS = boxs<T>(), RING = ring<T>();
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -405,8 +406,8 @@ __device__ __forceinline__ void sweep_cta(const SweepMaps &maps, const Geom &g, 
     t.j0 = by * zc.rows;
     const int L = g.L, M = g.M, N = g.N, XP = g.XP, PS = (int)g.PS;
     t.N = N;
-    t.k0 = zc.plane(c);
-    t.k1 = zc.plane(c + 1);
+    t.k0 = zc.plane(c) + (piece == Piece::LOWER ? 1 : 0);
+    t.k1 = piece == Piece::TOP ? t.k0 + 1 : zc.plane(c + 1);
     // rows: cells x = lane, lane + 32 of row w; column warp: one cell per lane, x = 64 of row `lane`.  A tile
     // has zc.rows rows, warp zc.rows computes the halo row and the warps between it and the column's idle.
     const bool column = w == 9;
@@ -509,6 +510,11 @@ __device__ __forceinline__ void sweep_cta(const SweepMaps &maps, const Geom &g, 
     carry_plane<0>(t, t.sm + (RING - 1) * NARR * BS);
     t.ex1 = t.ey1 = t.exn = t.eyn = t.ezn = dup<T>(T(0));
     t.bxo1 = t.byo1 = t.bxn = t.byn = t.acc = dup<T>(T(0));
+    if (piece == Piece::TOP && t.role == 0 && t.j < M) {  // the sum up to the plane below
+        const long long o = g.at(t.i, t.j, t.k1);
+        if (t.i < L && TCSEM_IN(o, g.total(), err)) t.acc.a = __ldcg(bz_new + o);
+        if (t.i + 32 < L && TCSEM_IN(o + 32, g.total(), err)) t.acc.b = __ldcg(bz_new + o + 32);
+    }
     async_shared_fence();
     __syncthreads();
     if (t.duty == 1 && ktop - (RING - 1) >= t.k0) load_stage(t, ktop - (RING - 1), RING - 1, air);

@@ -161,14 +161,14 @@ __global__ void __launch_bounds__(fs3::NT, sizeof(T) == 4 ? 2 : 1)
 // every slot of a batch in one launch: block b belongs to the slot whose range of idx holds it
 template <typename T>
 __global__ void __launch_bounds__(fs3::NT, sizeof(T) == 4 ? 2 : 1)
-    k_sweep_batched(const SweepSlot<T> *__restrict__ slots, const __grid_constant__ BatchIndex idx, int s, int c0) {
+    k_sweep_batched(const SweepSlot<T> *__restrict__ slots, const __grid_constant__ BatchIndex idx, int s, int c0, Piece piece) {
     const int q = idx.slot_of(blockIdx.x);
     const SweepSlot<T> &d = slots[q];
     const long st = (long)*d.step_base + s;
     if (st >= d.nsteps) return;
     const int lb = blockIdx.x - idx.off[q];
     const int bx = lb % d.tiles_x, rest = lb / d.tiles_x, by = rest % d.tiles_y, c = c0 + rest / d.tiles_y;
-    sweep_cta<T>(d.maps, d.g, d.tin, d.tout, d.ax, d.table[st], d.src, d.zc, bx, by, c, d.err);
+    sweep_cta<T>(d.maps, d.g, d.tin, d.tout, d.ax, d.table[st], d.src, d.zc, bx, by, c, d.err, AirAfterKernel(), piece, d.bz_new);
 }
 
 template <typename T>
@@ -189,10 +189,14 @@ void launch_fused_sweep(const SweepMaps &maps, const Geom &g, const T *tin, T *t
     cudaLaunchKernelEx(&cfg, k_sweep<T>, maps, g, tin, tout, ax, s, table, gate, src, zc, c0, rev ? 1 : 0, err);
 }
 
+// more than half of an SM's shared memory: one CTA per SM
+constexpr size_t kAloneBytes = 116 << 10;
 template <typename T>
-void launch_sweep_batched(const SweepSlot<T> *slots, const BatchIndex &idx, int s, int c0, int N_max, cudaStream_t st) {
+void launch_sweep_batched(const SweepSlot<T> *slots, const BatchIndex &idx, int s, int c0, int N_max, cudaStream_t st,
+                          Piece piece, bool spread) {
     if (idx.total() == 0) return;
-    k_sweep_batched<T><<<idx.total(), fs3::NT, fs3::smem_bytes_n<T>(N_max), st>>>(slots, idx, s, c0);
+    const size_t need = fs3::smem_bytes_n<T>(N_max);
+    k_sweep_batched<T><<<idx.total(), fs3::NT, spread && need < kAloneBytes ? kAloneBytes : need, st>>>(slots, idx, s, c0, piece);
 }
 int sweep_tiles_x(int L) { return (L + fs3::TX - 1) / fs3::TX; }
 int sweep_tiles_y(int M, int rows) { return (M + rows - 1) / rows; }
@@ -201,7 +205,8 @@ template <typename T> cudaError_t sweep_configure(int N) {
     const int sm = (int)fs3::smem_bytes_n<T>(N);
     cudaError_t e = cudaFuncSetAttribute(k_sweep<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
     if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(k_sweep_batched<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+    return cudaFuncSetAttribute(k_sweep_batched<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                sm < (int)kAloneBytes ? (int)kAloneBytes : sm);
 }
 template <typename T> size_t sweep_smem_bytes(int N) { return fs3::smem_bytes_n<T>(N); }
 template <typename T> int sweep_blocks_per_sm(int N) {
@@ -275,7 +280,7 @@ template <typename T> void launch_place(const Geom &g, const double *in, T *v, i
     template size_t sweep_smem_bytes<T>(int);                                                                      \
     template int sweep_blocks_per_sm<T>(int);                                                                      \
     template void launch_bz_consolidate<T>(const Geom &, T *, T *, const ZChunks &, cudaStream_t);             \
-    template void launch_sweep_batched<T>(const SweepSlot<T> *, const BatchIndex &, int, int, int, cudaStream_t);
+    template void launch_sweep_batched<T>(const SweepSlot<T> *, const BatchIndex &, int, int, int, cudaStream_t, Piece, bool);
 INST(float)
 INST(double)
 #undef INST
