@@ -91,7 +91,7 @@ template <typename T> static size_t smem_cols(const BoundaryDev<T> &bd) { return
 template <typename T> static size_t smem_inv(const BoundaryDev<T> &bd) { return rows_inv_layout(bd).total; }
 
 template <typename T> size_t boundary_smem_need(const BoundaryDev<T> &bd, int L) {
-    size_t a = smem_rows(bd, L), b = smem_cols(bd), c = smem_inv(bd);
+    size_t a = smem_rows(bd, L), b = cols_layout(bd).apart, c = smem_inv(bd);  // the limit on planes is that of regions apart
     return a > b ? (a > c ? a : c) : (b > c ? b : c);
 }
 

@@ -96,7 +96,7 @@ __device__ __forceinline__ T spline_out(const T *c, int npts, const T *y, int ys
 // the kernels and by the host for the launch size.  Every region starts on a
 // 16-byte boundary so the bulk copies can land in it.
 struct RowsFwdLayout { size_t bar, tw, tab, tabi, row, a, b, mb, total; };
-struct ColsLayout { size_t bar, tw, tab, tabi, col, gx, gy, a, b, mb, total; };
+struct ColsLayout { size_t bar, tw, tab, tabi, col, gx, gy, a, b, mb, total, apart; };  // apart: nothing on top of anything
 struct RowsInvLayout { size_t bar, tw, vx, vy, a, b, total; };
 
 template <typename T> __host__ __device__ inline RowsFwdLayout rows_fwd_layout(const BoundaryDev<T> &bd, int L) {
@@ -132,6 +132,7 @@ template <typename T> __host__ __device__ inline ColsLayout cols_layout(const Bo
     l.col = p; p += rnd16(bd.M * sizeof(C2<T>));
     l.mb = p; p += rnd16(4 * (size_t)bd.ry.nmax * sizeof(T));
     l.total = o > p ? o : p;
+    l.apart = o + (p - l.tab);
     return l;
 }
 template <typename T> __host__ __device__ inline RowsInvLayout rows_inv_layout(const BoundaryDev<T> &bd) {
