@@ -89,8 +89,8 @@ __device__ __forceinline__ double rcp64(double x) {
 }
 __device__ __forceinline__ Pair<double> rcp64(Pair<double> x) { return {rcp64(x.a), rcp64(x.b)}; }
 
-// per-thread state of the sweep; sweep_plane<PH>() advances one z-plane with PH = (ktop - k) mod 4, so ring
-// slots and buffer parities are compile-time constants
+// per-thread state of the sweep; sweep_plane() advances one z-plane: plane ktop - n reads the stage in slot n mod RING,
+// round n / RING, and the buffers of parity PAR = n mod 2
 template <typename T> struct SweepThread {
     T *sm;  // ring, then the new planes
     uint64_t *bars;
@@ -182,13 +182,13 @@ __device__ __forceinline__ void load_stage(const SweepThread<T> &t, int k, int q
 // planes' code has no condition on k but the two at the end of the ring.
 enum { FIRST, SECOND, INNER, LAST };
 
-template <typename T, int PH, int KIND, int ROLE, typename Air>
-__device__ __forceinline__ void sweep_plane(SweepThread<T> &t, int k, unsigned rp, const StepScalars<T> &s,
+template <typename T, int PAR, int KIND, int ROLE, typename Air>
+__device__ __forceinline__ void sweep_plane(SweepThread<T> &t, int k, int slot, int round, const StepScalars<T> &s,
                                             const Pair<T> *zt, const SourceTable<T> &src, const Air &air) {
     using namespace fs3;
     typedef Pair<T> P;
     constexpr int BS = boxs<T>(), RING = ring<T>();
-    constexpr int QE = PH & 1, QB = (PH + 1) & 1;
+    constexpr int QE = PAR, QB = PAR ^ 1;
     constexpr bool doB = (KIND == INNER || KIND == LAST) && ROLE != 3, doE = KIND != LAST && ROLE != 3;
     zt += 3 * (k - t.klow);  // dtb/dz, 1/(dz[k-1]+dz[k]), dz of plane k
     // Roles (one compiled copy each, FP64 only): the row warps update and store every component; the
@@ -219,7 +219,7 @@ __device__ __forceinline__ void sweep_plane(SweepThread<T> &t, int k, unsigned r
     if constexpr (doE) {
         t.ex1 = t.exn;
         t.ey1 = t.eyn;
-        const T *p0 = sm + PH % RING * NARR * BS;
+        const T *p0 = sm + slot * (NARR * BS);
         const int so = t.so;
         const P sx0 = t.sxk, sy0 = t.syk, sz0 = t.szk, bx0 = t.bxk, by0 = t.byk, bxj = t.bxj, byi = t.byi;
         carry_plane<ROLE>(t, p0);  // plane k-1, the next one up
@@ -308,9 +308,9 @@ __device__ __forceinline__ void sweep_plane(SweepThread<T> &t, int k, unsigned r
     }
     // stage k-1 is read by the next plane; a thread whose wait gave up does not wait again.  The last slot is
     // one phase ahead: it carried plane ktop's B and sigma first.
-    constexpr int NS = (PH + 1) % RING;
-    const unsigned parity = (RING == 4 ? rp ^ (unsigned)((PH + 1) >> 2) : (unsigned)((PH + 1) / RING) & 1u) ^ (NS == RING - 1 ? 1u : 0u);
-    if (KIND != LAST && k > t.k0 && !t.bad) t.bad = !mbar_wait_bounded(t.bars + NS, parity);
+    const int ns = (slot + 1) % RING;
+    const unsigned parity = (unsigned)(round + (ns == 0) + (ns == RING - 1)) & 1u;
+    if (KIND != LAST && k > t.k0 && !t.bad) t.bad = !mbar_wait_bounded(t.bars + ns, parity);
     async_shared_fence();  // the new planes are read by the TMA
     if (t.duty == 2) bulk_wait_read();  // ... which is done with the buffers the next plane writes
     __syncthreads();
@@ -328,7 +328,7 @@ __device__ __forceinline__ void sweep_plane(SweepThread<T> &t, int k, unsigned r
             }
             bulk_commit();
         } else if (KIND != LAST && k - RING >= t.k0) {  // the slot takes the stage RING planes up
-            load_stage(t, k - RING, PH % RING, air);
+            load_stage(t, k - RING, slot, air);
         }
     }
     // ---- Bz(k+1) = Bz(k+2) + dz (dBx/dx + dBy/dy), for the tile's own rows
@@ -351,38 +351,55 @@ template <typename T> __device__ __forceinline__ void set_offsets(SweepThread<T>
     }
 }
 
-// the z-march of one warp through the chunk, in the copy of the plane code for its role
-template <typename T, int ROLE, typename Air>
+// The z-march of one warp through the chunk, in the copy of the plane code for its role.  COPIES of the inner plane:
+// RING with the slots as constants, or 2 with the slot in a register and half of the code (256 x 256 x 160
+// 131.2 -> 128.7 us per step, in FP64 1348 -> 1336).  The batched and the cooperative kernel keep RING in FP32: there the
+// register is one too many (8 surveys of up to 152 x 131 x 112 170 -> 174 us, 64 x 64 x 48 19.2 -> 19.3).
+template <typename T, int ROLE, int COPIES, typename Air>
 __device__ __forceinline__ void sweep_march(SweepThread<T> &t, const StepScalars<T> &s, const Pair<T> *s_z,
                                             const SourceTable<T> &src, const T *s_oc, const Air &air) {
     using namespace fs3;
+    constexpr int RING = ring<T>();
+    static_assert(COPIES == 2 || (COPIES == 4 && RING == 4), "slots of the inner copies");
     const int k0 = t.k0;
-    sweep_plane<T, 0, FIRST, ROLE>(t, t.ktop, 0u, s, s_z, src, air);
+    sweep_plane<T, 0, FIRST, ROLE>(t, t.ktop, 0, 0, s, s_z, src, air);
     set_offsets(t, s_oc);
-    // the inner planes k = ktop - 2 .. k0 begin in phase 2; rp: parity of the ring round
+    // the inner planes k = ktop - 2 .. k0
     int k = t.ktop - 1;
-    sweep_plane<T, 1, SECOND, ROLE>(t, k, 0u, s, s_z, src, air);
-    unsigned rp = 0;
-    int left = 2;  // phase of the plane after the last inner one
-    while (--k >= k0) {
-        sweep_plane<T, 2, INNER, ROLE>(t, k, rp, s, s_z, src, air);
-        if (--k < k0) { left = 3; break; }
-        sweep_plane<T, 3, INNER, ROLE>(t, k, rp, s, s_z, src, air);
-        rp ^= 1u;
-        if (--k < k0) { left = 0; break; }
-        sweep_plane<T, 0, INNER, ROLE>(t, k, rp, s, s_z, src, air);
-        if (--k < k0) { left = 1; break; }
-        sweep_plane<T, 1, INNER, ROLE>(t, k, rp, s, s_z, src, air);
+    sweep_plane<T, 1, SECOND, ROLE>(t, k, 1 % RING, 1 / RING, s, s_z, src, air);
+    if constexpr (COPIES == 2) {
+        int n = 2;  // planes done
+        while (--k >= k0) {
+            sweep_plane<T, 0, INNER, ROLE>(t, k, n % RING, n / RING, s, s_z, src, air);
+            n++;
+            if (--k < k0) break;
+            sweep_plane<T, 1, INNER, ROLE>(t, k, n % RING, n / RING, s, s_z, src, air);
+            n++;
+        }
+        if (n & 1) sweep_plane<T, 1, LAST, ROLE>(t, k, n % RING, n / RING, s, s_z, src, air);
+        else sweep_plane<T, 0, LAST, ROLE>(t, k, n % RING, n / RING, s, s_z, src, air);
+    } else {
+        int round = 0, left = 2;  // slot of the plane after the last inner one
+        while (--k >= k0) {
+            sweep_plane<T, 0, INNER, ROLE>(t, k, 2, round, s, s_z, src, air);
+            if (--k < k0) { left = 3; break; }
+            sweep_plane<T, 1, INNER, ROLE>(t, k, 3, round, s, s_z, src, air);
+            round ^= 1;
+            if (--k < k0) { left = 0; break; }
+            sweep_plane<T, 0, INNER, ROLE>(t, k, 0, round, s, s_z, src, air);
+            if (--k < k0) { left = 1; break; }
+            sweep_plane<T, 1, INNER, ROLE>(t, k, 1, round, s, s_z, src, air);
+        }
+        if (left == 0) sweep_plane<T, 0, LAST, ROLE>(t, k, 0, round, s, s_z, src, air);
+        else if (left == 1) sweep_plane<T, 1, LAST, ROLE>(t, k, 1, round, s, s_z, src, air);
+        else if (left == 2) sweep_plane<T, 0, LAST, ROLE>(t, k, 2, round, s, s_z, src, air);
+        else sweep_plane<T, 1, LAST, ROLE>(t, k, 3, round, s, s_z, src, air);
     }
-    if (left == 0) sweep_plane<T, 0, LAST, ROLE>(t, k, rp, s, s_z, src, air);
-    else if (left == 1) sweep_plane<T, 1, LAST, ROLE>(t, k, rp, s, s_z, src, air);
-    else if (left == 2) sweep_plane<T, 2, LAST, ROLE>(t, k, rp, s, s_z, src, air);
-    else sweep_plane<T, 3, LAST, ROLE>(t, k, rp, s, s_z, src, air);
 }
 
 // one CTA of the sweep: tile (bx, by) of z-chunk c (or a piece of the only chunk) with the step scalars s.  FRESH: the chunk
 // totals tin may have been written by another CTA of the same launch (persistent schedule).
-template <typename T, bool FRESH = false, typename Air = AirAfterKernel>
+template <typename T, bool FRESH = false, int COPIES = fs3::ring<T>(), typename Air = AirAfterKernel>
 __device__ __forceinline__ void sweep_cta(const SweepMaps &maps, const Geom &g, const T *__restrict__ tin,
                                           T *__restrict__ tout, const Axis<T> &ax, StepScalars<T> s,
                                           const SourceTable<T> &src, const ZChunks &zc, int bx, int by, int c, int *err,
@@ -527,12 +544,12 @@ __device__ __forceinline__ void sweep_cta(const SweepMaps &maps, const Geom &g, 
     // (5 % faster).  FP32 runs one copy in every warp: three copies of its loop made the sweep 40 %
     // slower (measured; presumably the larger loop no longer fits the instruction cache).
     if constexpr (sizeof(T) == 8) {
-        if (t.role == 0) sweep_march<T, 0>(t, s, s_z, src, s_oc, air);
-        else if (t.role == 1) sweep_march<T, 1>(t, s, s_z, src, s_oc, air);
-        else if (t.role == 2) sweep_march<T, 2>(t, s, s_z, src, s_oc, air);
-        else sweep_march<T, 3>(t, s, s_z, src, s_oc, air);
+        if (t.role == 0) sweep_march<T, 0, COPIES>(t, s, s_z, src, s_oc, air);
+        else if (t.role == 1) sweep_march<T, 1, COPIES>(t, s, s_z, src, s_oc, air);
+        else if (t.role == 2) sweep_march<T, 2, COPIES>(t, s, s_z, src, s_oc, air);
+        else sweep_march<T, 3, COPIES>(t, s, s_z, src, s_oc, air);
     } else {
-        sweep_march<T, 0>(t, s, s_z, src, s_oc, air);
+        sweep_march<T, 0, COPIES>(t, s, s_z, src, s_oc, air);
     }
     // the last plane's Bz, in the buffer of its parity
     async_shared_fence();

@@ -155,7 +155,7 @@ __global__ void __launch_bounds__(fs3::NT, sizeof(T) == 4 ? 2 : 1)
         s = table[st];
     }
     const int c = cbase + (int)(rev ? gridDim.z - 1 - blockIdx.z : blockIdx.z);
-    sweep_cta<T>(maps, g, tin, tout, ax, s, src, zc, blockIdx.x, blockIdx.y, c, err);
+    sweep_cta<T, false, 2>(maps, g, tin, tout, ax, s, src, zc, blockIdx.x, blockIdx.y, c, err);
 }
 
 // every slot of a batch in one launch: block b belongs to the slot whose range of idx holds it
