@@ -441,7 +441,7 @@ template <typename T> struct SimImpl : SimBase {
             // run at two lanes per clock on the SMs left free, after about 25 us of latency, or after the sweep.
             // Measured, us per step with this rule and with 8 rows and one chunk more than 85 % of the SMs hold
             // (chunks of 8 planes or more): 44 x 38 x 27 49 and 145, 64 x 64 x 48 78 and 116, 160 x 56 x 40 131 and
-            // 139, 128 x 128 x 96 228 and 265, 187 x 121 x 101 386 and 594, 256 x 256 x 160 1349 and 1583.
+            // 139, 128 x 128 x 96 228 and 265, 187 x 121 x 101 386 and 594, 256 x 256 x 160 1336 and 1583.
             const double work = (((m.M + 1) / 2 + bd.S) * fft_ops(bd.px) + 3.0 * bd.H * fft_ops(bd.py)) / 4140.0;
             double best = 1e30;
             int lower = 1;

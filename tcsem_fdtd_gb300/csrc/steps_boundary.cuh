@@ -86,11 +86,6 @@ template <typename T> inline void products_bind(Products<T> &d, T *const p[kProd
     d.Cxc = p[5]; d.Cxs = p[6]; d.Cyc = p[7]; d.Cys = p[8]; d.Dx = p[9]; d.Dy = p[10];
     d.F = p[11]; d.V = p[12];
 }
-// multiply-adds of one boundary step
-template <typename T> inline double products_fma(const Products<T> &d) {
-    return (double)d.nc * ((double)d.L * d.M + (double)(d.Mh + d.Rx + d.Ry) * d.M1 + (double)d.M * (d.L + 1) +
-                           (double)(d.M + 1) * d.L);
-}
 template <typename T> inline int tiles_fwd(const Products<T> &d) {
     return up(d.nc, kTabN) * (d.fold ? up(d.Mh, kFwdJ / 2) : up(d.M, kFwdJ));
 }
