@@ -87,7 +87,11 @@ __global__ void k_bilinear_b(const BoundarySlot<T> *__restrict__ slots, const __
 }
 
 template <typename T> static size_t smem_rows(const BoundaryDev<T> &bd, int L) { return rows_fwd_layout(bd, L).total; }
-template <typename T> static size_t smem_cols(const BoundaryDev<T> &bd) { return cols_layout(bd).total; }
+template <typename T> static size_t smem_cols(const BoundaryDev<T> &bd) {
+    const size_t t = cols_layout(bd).total;
+    return t > bd.cols_pad ? t : bd.cols_pad;
+}
+template <typename T> size_t cols_apart(const BoundaryDev<T> &bd) { return cols_layout(bd).apart; }
 template <typename T> static size_t smem_inv(const BoundaryDev<T> &bd) { return rows_inv_layout(bd).total; }
 
 template <typename T> size_t boundary_smem_need(const BoundaryDev<T> &bd, int L) {
@@ -99,7 +103,7 @@ template <typename T> cudaError_t boundary_configure(const BoundaryDev<T> &bd, i
     cudaError_t e;
     e = cudaFuncSetAttribute(k_rows_fwd<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_rows(bd, L));
     if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(k_cols<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_cols(bd));
+    e = cudaFuncSetAttribute(k_cols<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cols_apart(bd));
     if (e != cudaSuccess) return e;
     return cudaFuncSetAttribute(k_rows_inv<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_inv(bd));
 }
@@ -165,6 +169,7 @@ void launch_boundary(const BoundaryDev<T> &bd, const Geom &g, const T *bz, const
 }
 
 #define INST(T)                                                                                            \
+    template size_t cols_apart<T>(const BoundaryDev<T> &);                                                        \
     template size_t boundary_smem_need<T>(const BoundaryDev<T> &, int);                                   \
     template cudaError_t boundary_configure<T>(const BoundaryDev<T> &, int);                              \
     template void launch_boundary<T>(const BoundaryDev<T> &, const Geom &, const T *, const T *, int, T *, T *,  \

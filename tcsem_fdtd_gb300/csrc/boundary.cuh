@@ -33,6 +33,7 @@ template <typename T> struct AxisRemap {
 };
 
 template <typename T> struct BoundaryDev {
+    size_t cols_pad = 0;  // shared memory that a block of the column stage asks for at least
     // plane geometry: the transforms have L1 x M1 points; the uniform grid (Lu x Mu points)
     // sits at offset (DL, DM) in them.  Without padding Lu = L1, Mu = M1, DL = DM = 0; with
     // padding the points outside the grid taper each row (column) from its edge values to
@@ -81,6 +82,7 @@ struct BoundaryBlocks {
 
 namespace tcsem {
 template <typename T> size_t boundary_smem_need(const BoundaryDev<T> &bd, int L);
+template <typename T> size_t cols_apart(const BoundaryDev<T> &bd);  // of the column stage with no region on top of another
 template <typename T> cudaError_t boundary_configure(const BoundaryDev<T> &bd, int L);
 // pdl: the last three kernels may start while their predecessor finishes (programmatic
 // dependent launch); off where the chain runs beside a long sweep whose CTAs need the slots

@@ -359,6 +359,10 @@ template <typename T> struct SimImpl : SimBase {
         cudaEventDestroy(e1);
         CK(cudaGetLastError());
         overlap_pdl = t_bnd >= 0.5f * t_sweep;
+        // Where the boundary takes much longer than the sweep, its column blocks must not crowd on the SMs that the
+        // sweep leaves at first: two per SM there, and the rest everywhere once the sweep is done (247 x 117 x 49 with
+        // a 687 x 557 plane, the boundary 110 us and the sweep 21: 175 us per step with three, 156 with two).
+        if (t_bnd > 1.5f * t_sweep) bd.cols_pad = cols_apart(bd);
         zero_state();
     }
 
