@@ -199,6 +199,7 @@ __device__ __forceinline__ void rows_fwd_cta(const BoundaryDev<T> &bd, const T *
                        bi = (unsigned)rnd16(R.nI * sizeof(int));
         mbar_init(bar, 1);
         mbar_init_fence();
+        async_shared_fence();  // the memory may hold an earlier unit's ordinary stores (persistent schedule)
         mbar_expect_tx(bar, btw + bt + bi);
         bulk_load(tw, bd.twx, btw, bar);
         bulk_load(tab, R.tabT, bt, bar);
@@ -286,6 +287,7 @@ __device__ __forceinline__ void cols_cta(const BoundaryDev<T> &bd, int blk) {
         const bool okc = TCSEM_IN((long long)kx * bd.Mp + bc / sizeof(C2<T>) - 1, (long long)bd.H * bd.Mp, bd.err);
         mbar_init(bar, 1);
         mbar_init_fence();
+        async_shared_fence();
         mbar_expect_tx(bar, btw + bt + bi + (okc ? bc : 0u) + 2 * bg);
         bulk_load(tw, bd.twy, btw, bar);
         bulk_load(tab, R.tabT, bt, bar);
@@ -360,6 +362,7 @@ __device__ __forceinline__ void rows_inv_cta(const BoundaryDev<T> &bd, int blk) 
         const bool okv = TCSEM_IN((long long)s * bd.Hp + bv / sizeof(C2<T>) - 1, (long long)bd.S * bd.Hp, bd.err);
         mbar_init(bar, 1);
         mbar_init_fence();
+        async_shared_fence();
         mbar_expect_tx(bar, btw + (okv ? 2 * bv : 0u));
         bulk_load(tw, bd.twx, btw, bar);
         pdl_wait_prev();  // VX and VY are the previous kernel's output

@@ -176,6 +176,7 @@ template <typename T, int J> struct Tile {
         if (threadIdx.x != 0) return;
         for (int q = 0; q < l.nslot; q++) mbar_init(bars + q, 1);
         mbar_init_fence();
+        async_shared_fence();  // the product before left ordinary stores where the copies land
         for (int c = 0; c < l.nslot; c++) load_chunk(c);
     }
     // all threads: the sums of this lane's share, into slots[warp][J][32]; false: a copy did not arrive

@@ -496,6 +496,7 @@ __device__ __forceinline__ void sweep_cta(const SweepMaps &maps, const Geom &g, 
     __syncthreads();
     if (t.duty == 1) {  // B and sigma of plane ktop through the last slot, the first stages into the others
         uint64_t *b = t.bars + RING - 1;
+        async_shared_fence();  // another role's ordinary stores, where CTAs outlive one tile
         mbar_expect_tx(b, (unsigned)(3 * BOX * sizeof(T)));
         for (int a : {ABX, ABY, ASG})
             tma_load_3d(t.sm + ((RING - 1) * NARR + a) * BS, maps.m + a, t.i0, t.j0, ktop + 1, b);
