@@ -285,6 +285,13 @@ tcsem_status tcsem_selftest_bounded_wait(int device, int polls, int *gave_up);
  * (or tcsem_batch_traces of a slot) returns TCSEM_ERR_CUDA. */
 tcsem_status tcsem_selftest_queue_wait(int device, long long wait_ns, int *gave_up);
 
+/* Self-test of the sweep's bounded waits (no counterpart in the reference): one sweep from the
+ * handle's fields whose waits for copies all give up at once, as if the copies had not arrived.
+ * *gave_up is 1 when the error word says so.  A tile whose wait gave up loads nothing more into
+ * the slot it waited for: *loaded, the tiles that went on to the last plane, is 0.  The handle's
+ * fields and its run in progress are as before. */
+tcsem_status tcsem_selftest_copy_wait(tcsem_sim_t *sim, int *gave_up, int *loaded);
+
 #ifdef __cplusplus
 }
 #endif

@@ -112,6 +112,7 @@ def library():
         "tcsem_timed_advance": (i, [vp, l_, dp]),
         "tcsem_selftest_bounded_wait": (i, [i, i, ip]),
         "tcsem_selftest_queue_wait": (i, [i, C.c_longlong, ip]),
+        "tcsem_selftest_copy_wait": (i, [vp, ip, ip]),
     }
     sig.update({
         "tcsem_batch_create": (i, [C.POINTER(Opts), C.c_size_t, C.POINTER(vp)]),
@@ -342,6 +343,12 @@ class Simulation:
         ms = C.c_double()
         self._check(library().tcsem_timed_advance(self._h, nsteps, C.byref(ms)))
         return ms.value
+
+    def selftest_copy_wait(self):
+        """tcsem_selftest_copy_wait: (whether the sweep's waits gave up, tiles that went on loading all the same)."""
+        g, n = C.c_int(0), C.c_int(0)
+        self._check(library().tcsem_selftest_copy_wait(self._h, C.byref(g), C.byref(n)))
+        return bool(g.value), n.value
 
     def time_steps(self, itx, nsteps):
         """Device time (ms) of `nsteps` captured steps, and of one sweep / one boundary pass."""

@@ -201,6 +201,13 @@ tcsem_status tcsem_selftest_bounded_wait(int device, int polls, int *gave_up) {
     return st;
 }
 
+tcsem_status tcsem_selftest_copy_wait(tcsem_sim_t *s, int *gave_up, int *loaded) {
+    return guard(s, [&](SimBase &b) {
+        if (!gave_up || !loaded) throw Error(TCSEM_ERR_INVALID, "null output");
+        b.selftest_copy_wait(gave_up, loaded);
+    });
+}
+
 tcsem_status tcsem_write_bout(tcsem_sim_t *s, int itx, const double *t, const char *path) {
     return guard(s, [&](SimBase &b) {
         if (!t || !path) throw Error(TCSEM_ERR_INVALID, "null argument");

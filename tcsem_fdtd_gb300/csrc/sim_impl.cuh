@@ -32,6 +32,7 @@
 #include "check.cuh"
 #include "kernels.cuh"
 #include "rx.cuh"
+#include "selftest.cuh"
 #include "setup.h"
 #include "steps.cuh"
 #include "tcsem.h"
@@ -135,6 +136,7 @@ struct SimBase {
     virtual void time_steps(int itx, long n, double *tot, double *sweep, double *bnd) = 0;
     virtual void timed_advance(long n, double *ms) = 0;
     virtual void check_error() = 0;
+    virtual void selftest_copy_wait(int *gave_up, int *loaded) = 0;
     virtual void save_state(const char *path) = 0;
     virtual void load_state(const char *path) = 0;
     size_t field_count(int comp) const {
@@ -762,6 +764,26 @@ template <typename T> struct SimImpl : SimBase {
                 throw Error(TCSEM_ERR_CUDA, "a kernel index fell outside its array (bounds-checked build)");
             throw Error(TCSEM_ERR_CUDA, "a bounded wait in a kernel gave up (a bulk copy did not arrive)");
         }
+    }
+    // a sweep from the current set whose waits for copies give up at once
+    void selftest_copy_wait(int *gave_up, int *loaded) override {
+        if (model.N < 8) throw Error(TCSEM_ERR_INVALID, "the self-test needs at least 8 planes");
+        need_tx();
+        const int b = cur;
+        DevMem n;
+        n.alloc(sizeof(int));
+        dzero(n.p, sizeof(int));
+        CK(launch_sweep_lost<T>(maps[b], g, tot[b].as<T>(), tot[b ^ 1].as<T>(), ax,
+                                scal(sched.lam[0], sched.dt1[0], sched.dtB[0], 0.0), src, zc.rows, errw.as<int>(), n.as<int>(),
+                                stream));
+        int h = 0;
+        d2h(&h, errw.p, sizeof h);
+        dzero(errw.p, sizeof h);
+        *gave_up = h == 1;
+        d2h(loaded, n.p, sizeof h);
+        for (int c = 0; c < 6; c++)  // the other set has what the sweep made of nothing
+            CK(cudaMemcpyAsync(fld[b ^ 1][c].p, fld[b][c].p, fld[b][c].n, cudaMemcpyDeviceToDevice, stream));
+        CK(cudaStreamSynchronize(stream));
     }
     void sweep(int b, StepScalars<T> s, const StepScalars<T> *table, StepGate gate, int c0 = 0, int c1 = -1,
                cudaStream_t st = nullptr, bool pdl = false) {

@@ -61,6 +61,10 @@ template <typename T> struct Sync {
         }
         return !__syncthreads_or(!ok);
     }
+    // all threads, a copy did not arrive (err is set): the other CTAs leave at their next wait
+    __device__ __forceinline__ void give_up() const {
+        if (threadIdx.x == 0) atomicExch(a.ctl + kStAbort, 1);
+    }
     // all threads: the end of step s of this launch
     __device__ __forceinline__ bool step_end(int s) const {
         arrive<true>(a.ctl + kStArrive);
@@ -71,6 +75,7 @@ template <typename T> struct Sync {
 // the sweep's copying thread before the air plane; when it gives up the sweep finishes on the old
 // plane and its CTA leaves at the next wait
 template <typename T> struct AirFlag {
+    static constexpr int kPolls = AirAfterKernel::kPolls;
     Sync<T> s;
     int target;
     __device__ __forceinline__ void operator()() const {
@@ -78,7 +83,7 @@ template <typename T> struct AirFlag {
         fence_proxy_async_global();
     }
 };
-// a product before it reads the one before (word; nothing to wait for without one)
+// a product before it reads the one before (word; nothing to wait for without one); ok: the CTA goes on
 template <typename T> struct After {
     Sync<T> s;
     const int *word;
@@ -86,6 +91,11 @@ template <typename T> struct After {
     bool *ok;
     __device__ __forceinline__ void operator()() const {
         if (word) *ok = s.template wait<false>(word, target) && *ok;
+    }
+    // a copy did not arrive: the CTA leaves at the end of the step, the others at a wait
+    __device__ __forceinline__ void lost() const {
+        *ok = false;
+        s.give_up();
     }
 };
 
@@ -105,8 +115,10 @@ __global__ void __launch_bounds__(fs3::NT, 2) k_steps(const __grid_constant__ St
             for (int c = r < a.march ? r + 1 : a.zc.n;; c += a.march) {
                 const bool top = c >= a.zc.n;
                 if (top && r != a.march - 1 + a.own) break;
-                sweep_cta<T, true>(a.maps[b], a.g, a.tot[b], a.tot[b ^ 1], a.ax, a.table[a.step0 + s], a.src, a.zc,
-                                   tile % a.tiles_x, tile / a.tiles_x, top ? 0 : c, a.err, AirFlag<T>{sy, (s + 1) * a.nbnd});
+                const bool ok = sweep_cta<T, true>(a.maps[b], a.g, a.tot[b], a.tot[b ^ 1], a.ax, a.table[a.step0 + s], a.src,
+                                                   a.zc, tile % a.tiles_x, tile / a.tiles_x, top ? 0 : c, a.err,
+                                                   AirFlag<T>{sy, (s + 1) * a.nbnd});
+                if (!ok) return sy.give_up();
                 __syncthreads();
                 if (threadIdx.x == 0) {
                     uint64_t *ring = reinterpret_cast<uint64_t *>(smem_raw + fs3::bars_offset<T>());

@@ -203,6 +203,7 @@ template <typename T, int J> struct Tile {
         };
         const T *x0 = xrow(jq) + w * SH;
         bool ok = true;
+        int loaded = l.nslot;  // chunks thread 0 has asked for
         for (int c = 0; c < l.nchunk; c++) {
             ok = mbar_wait_bounded(bars + c % l.nslot, (unsigned)(c / l.nslot) & 1u) && ok;
             const T *t = slots + ((size_t)(c % l.nslot) * CHUNK + w * SH) * kTabN + 4 * nq;
@@ -232,18 +233,18 @@ template <typename T, int J> struct Tile {
 #pragma unroll
                 for (int j = 0; j < NJ; j++) acc[0][j] = acc[1][j] = dup<T>(T(0));
             }
-            if (c + l.nslot < l.nchunk) {  // the slot takes its next chunk
+            if (c + l.nslot < l.nchunk) {  // the slot takes its next chunk, once the loading thread has seen it filled
                 __syncthreads();
-                if (threadIdx.x == 0) {
+                if (threadIdx.x == 0 && ok) {
                     async_shared_fence();
-                    load_chunk(c + l.nslot);
+                    load_chunk(loaded++);
                 }
             }
         }
         if (__syncthreads_or(!ok)) {  // record it, let the copies land, leave together
             if (threadIdx.x == 0) {
                 atomicExch(err, 1);
-                for (int c = max(0, l.nchunk - l.nslot); c < l.nchunk; c++)
+                for (int c = loaded - l.nslot; c < loaded; c++)
                     mbar_wait_bounded(bars + c % l.nslot, (unsigned)(c / l.nslot) & 1u);
             }
             __syncthreads();
@@ -275,7 +276,8 @@ template <typename T, int J> struct Tile {
 };
 
 // columns of every grid row, as even and odd parts in y.  Plane 0 of Bz is chunk-partial: the totals of the
-// chunks below are added as it is loaded.  wait(): before the fields of the step before are read.
+// chunks below are added as it is loaded.  wait(): before the fields of the step before are read;
+// wait.lost(): a copy of the table did not arrive.
 template <typename T, typename Wait>
 __device__ __forceinline__ void forward_x(const Products<T> &d, const T *__restrict__ bz, const T *__restrict__ tot, int nch,
                                           const Geom &g, int blk, const Wait &wait) {
@@ -328,6 +330,8 @@ __device__ __forceinline__ void forward_x(const Products<T> &d, const T *__restr
             }
             *reinterpret_cast<Vec4<T> *>(d.F + (size_t)c * d.ldF + odd * d.oFo + j) = o;
         }
+    } else {
+        wait.lost();
     }
     __syncthreads();
     if (threadIdx.x == 0) t.retire();
@@ -375,6 +379,8 @@ __device__ __forceinline__ void inverse_x(const Products<T> &d, T *bx, T *by, co
             else
                 for (int q = 0; q < nn - i; q++) dst[q] = o.v[q];
         }
+    } else {
+        wait.lost();
     }
     __syncthreads();
     if (threadIdx.x == 0) t.retire();

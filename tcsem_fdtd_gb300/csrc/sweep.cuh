@@ -59,6 +59,7 @@ enum { AEX = 0, AEY, AEZ, ABX, ABY, ABZ, ASG };
 constexpr int XCOL = 9 * TX, XBUF = 10 * TX, SBUF = BY * TX;
 enum { XEZ = 0, XBX, XBY };
 enum { SEX = 0, SEY, SBZ };
+constexpr int kLost = 1 << 30;  // above every plane's number
 template <typename T> __host__ __device__ constexpr int xoff(int a, int q) { return ring<T>() * NARR * boxs<T>() + (2 * a + q) * XBUF; }
 template <typename T> __host__ __device__ constexpr int soff(int a, int q) { return xoff<T>(3, 0) + (3 * q + a) * SBUF; }
 // byte offset of the ring's mbarriers and the source planes; then the z tables
@@ -97,9 +98,9 @@ template <typename T> struct SweepThread {
     int *s_src;  // first and last plane with a source segment in the tile
     const SweepMaps *maps;
     int j, N, k0, k1, klow, ktop, i0, j0;
+    int kend;     // last plane whose stage the thread waits for, or loads: k0, or kLost + the stage at which it gave up
     int role;     // 0: a row of the tile, 1: the +y halo row, 2: the +x halo column, 3: none (warp-uniform)
     int duty;     // 1: the thread issues the loads (a lane of warp 8), 2: the stores (of the +x warp)
-    bool bad;     // a copy did not arrive
     bool src;     // a source segment touches the tile in this step
     int so, xo, xd, xr, i;         // first cell: in the box, in the new planes; its +y and the second one's +x neighbour; x index
     // which components of the cells are updated: bits 0, 1 Ex and By, bits 2, 3 Ey and Bx (both: Ez too);
@@ -157,6 +158,7 @@ template <int ROLE, typename T> __device__ __forceinline__ void carry_plane(Swee
 // previous kernel on the stream (a top chunk launched early, programmatic dependent launch after the
 // boundary's last stage, waits for it there and not before; no-op without the launch attribute).
 struct AirAfterKernel {
+    static constexpr int kPolls = 1 << 20;  // of a copy, before the wait for it gives up
     __device__ __forceinline__ void operator()() const { pdl_wait_prev(); }
 };
 // the loading thread: stage k into slot q
@@ -306,11 +308,11 @@ __device__ __forceinline__ void sweep_plane(SweepThread<T> &t, int k, int slot, 
         if constexpr (rY) rput<ROLE>(sm + xoff<T>(XBX, QB), t.xo, t.bxn);
         if constexpr (rX) rput<ROLE>(sm + xoff<T>(XBY, QB), t.xo, t.byn);
     }
-    // stage k-1 is read by the next plane; a thread whose wait gave up does not wait again.  The last slot is
-    // one phase ahead: it carried plane ktop's B and sigma first.
+    // stage k-1 is read by the next plane; a thread whose wait gave up waits for no other, and loads none.  The last
+    // slot is one phase ahead: it carried plane ktop's B and sigma first.
     const int ns = (slot + 1) % RING;
     const unsigned parity = (unsigned)(round + (ns == 0) + (ns == RING - 1)) & 1u;
-    if (KIND != LAST && k > t.k0 && !t.bad) t.bad = !mbar_wait_bounded(t.bars + ns, parity);
+    if (KIND != LAST && k > t.kend && !mbar_wait_bounded(t.bars + ns, parity, Air::kPolls)) t.kend = kLost + k - 1;
     async_shared_fence();  // the new planes are read by the TMA
     if (t.duty == 2) bulk_wait_read();  // ... which is done with the buffers the next plane writes
     __syncthreads();
@@ -327,7 +329,7 @@ __device__ __forceinline__ void sweep_plane(SweepThread<T> &t, int k, int slot, 
                 if (k + 2 < t.k1) tma_store_3d(t.maps->o + 5, sm + soff<T>(SBZ, QB), t.i0, t.j0, k + 2);
             }
             bulk_commit();
-        } else if (KIND != LAST && k - RING >= t.k0) {  // the slot takes the stage RING planes up
+        } else if (KIND != LAST && k - RING >= t.kend) {  // the slot takes the stage RING planes up
             load_stage(t, k - RING, slot, air);
         }
     }
@@ -398,9 +400,10 @@ __device__ __forceinline__ void sweep_march(SweepThread<T> &t, const StepScalars
 }
 
 // one CTA of the sweep: tile (bx, by) of z-chunk c (or a piece of the only chunk) with the step scalars s.  FRESH: the chunk
-// totals tin may have been written by another CTA of the same launch (persistent schedule).
+// totals tin may have been written by another CTA of the same launch (persistent schedule).  False (for all threads): a
+// copy did not arrive; it is recorded in err, and no copy is in flight.
 template <typename T, bool FRESH = false, int COPIES = fs3::ring<T>(), typename Air = AirAfterKernel>
-__device__ __forceinline__ void sweep_cta(const SweepMaps &maps, const Geom &g, const T *__restrict__ tin,
+__device__ __forceinline__ bool sweep_cta(const SweepMaps &maps, const Geom &g, const T *__restrict__ tin,
                                           T *__restrict__ tout, const Axis<T> &ax, StepScalars<T> s,
                                           const SourceTable<T> &src, const ZChunks &zc, int bx, int by, int c, int *err,
                                           const Air &air = Air(), Piece piece = Piece::WHOLE,
@@ -523,8 +526,7 @@ __device__ __forceinline__ void sweep_cta(const SweepMaps &maps, const Geom &g, 
         s_oc[e] = o;
         s_oc1[e] = o1;
     }
-    t.bad = !mbar_wait_bounded(t.bars + RING - 1, 0u);
-    if (!t.bad) t.bad = !mbar_wait_bounded(t.bars + 0, 0u);
+    t.kend = mbar_wait_bounded(t.bars + RING - 1, 0u) && mbar_wait_bounded(t.bars + 0, 0u) ? t.k0 : kLost + ktop;
     carry_plane<0>(t, t.sm + (RING - 1) * NARR * BS);
     t.ex1 = t.ey1 = t.exn = t.eyn = t.ezn = dup<T>(T(0));
     t.bxo1 = t.byo1 = t.bxn = t.byn = t.acc = dup<T>(T(0));
@@ -535,7 +537,7 @@ __device__ __forceinline__ void sweep_cta(const SweepMaps &maps, const Geom &g, 
     }
     async_shared_fence();
     __syncthreads();
-    if (t.duty == 1 && ktop - (RING - 1) >= t.k0) load_stage(t, ktop - (RING - 1), RING - 1, air);
+    if (t.duty == 1 && ktop - (RING - 1) >= t.kend) load_stage(t, ktop - (RING - 1), RING - 1, air);
 
     // Bz offsets of the first plane: ktop is the halo plane k1 of the chunk below (its offsets) or the
     // zero bottom; every later plane lies in this chunk
@@ -554,22 +556,28 @@ __device__ __forceinline__ void sweep_cta(const SweepMaps &maps, const Geom &g, 
     }
     // the last plane's Bz, in the buffer of its parity
     async_shared_fence();
-    const bool bad = __syncthreads_or(t.bad);
+    const bool bad = __syncthreads_or(t.kend >= kLost);
     if (t.duty == 2) {
         tma_store_3d(maps.o + 5, t.sm + ((ktop - klow) & 1 ? soff<T>(SBZ, 1) : soff<T>(SBZ, 0)), t.i0, t.j0, t.k0);
         bulk_commit();
         bulk_wait_all();
     }
-    if (bad) {  // a copy did not arrive: record it and let the last planes land
+    if (bad) {  // a copy did not arrive: record it and let those in flight land
         if (t.duty == 1) {
             atomicExch(err, 1);
-            for (int k = t.k0; k <= ktop && k < t.k0 + RING; k++) {
-                const int n = ktop - k;  // stages land in order: slot n % RING, round n / RING
-                mbar_wait_bounded(t.bars + n % RING, (unsigned)(n / RING + (n % RING == RING - 1)) & 1u);
+            // Unless this thread gave up, it has seen every stage land.  Having given up on stage `lost` it loaded no
+            // more: the RING - 1 stages from that one on were under way (and at the first one, ktop's B and sigma).
+            if (t.kend >= kLost) {
+                const int lost = t.kend - kLost;
+                if (lost == ktop) mbar_wait_bounded(t.bars + RING - 1, 0u);
+                for (int k = lost; k > lost - (RING - 1) && k >= t.k0; k--) {
+                    const int n = ktop - k;  // slot n % RING, round n / RING
+                    mbar_wait_bounded(t.bars + n % RING, (unsigned)(n / RING + (n % RING == RING - 1)) & 1u);
+                }
             }
         }
         __syncthreads();
-        return;
+        return false;
     }
     if (zc.n > 1 && t.role == 0) {
         const T a[2] = {t.acc.a, t.acc.b};
@@ -579,6 +587,7 @@ __device__ __forceinline__ void sweep_cta(const SweepMaps &maps, const Geom &g, 
             if (t.j < M && t.i + 32 * q < L && TCSEM_IN(o, zc.n * PS, err)) tout[o] = a[q];
         }
     }
+    return true;
 }
 
 }  // namespace tcsem
