@@ -359,7 +359,12 @@ template <typename T> struct BatchImpl : BatchBase {
             launch_rx_batched<T>(drs[p].as<RxSlot<T>>(), g0.irs, s, stream);
         }
         launch_advance_all(counters.as<int>(), n, gsteps, stream);
+        const cudaError_t refused = cudaGetLastError();  // of a launch: the graph lacks it
         cudaError_t e = cudaStreamEndCapture(stream, &graph);
+        if (e == cudaSuccess && refused != cudaSuccess) {
+            cudaGraphDestroy(graph);
+            e = refused;
+        }
         if (e != cudaSuccess) throw Error(TCSEM_ERR_CUDA, std::string("batch graph capture: ") + cudaGetErrorString(e));
         e = cudaGraphInstantiateWithFlags(&gexec, graph, cudaGraphInstantiateFlagUseNodePriority);
         cudaGraphDestroy(graph);

@@ -100,12 +100,10 @@ template <typename T> size_t boundary_smem_need(const BoundaryDev<T> &bd, int L)
 }
 
 template <typename T> cudaError_t boundary_configure(const BoundaryDev<T> &bd, int L) {
-    cudaError_t e;
-    e = cudaFuncSetAttribute(k_rows_fwd<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_rows(bd, L));
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(k_cols<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cols_apart(bd));
-    if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(k_rows_inv<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_inv(bd));
+    cudaError_t e = allow_shared(k_rows_fwd<T>, smem_rows(bd, L));
+    if (e == cudaSuccess) e = allow_shared(k_cols<T>, cols_apart(bd));
+    if (e == cudaSuccess) e = allow_shared(k_rows_inv<T>, smem_inv(bd));
+    return e;
 }
 
 template <typename T> BoundaryBlocks boundary_blocks(const BoundaryDev<T> &bd, const Geom &g) {
@@ -121,10 +119,9 @@ template <typename T> BoundaryBlocks boundary_blocks(const BoundaryDev<T> &bd, c
 }
 
 template <typename T> cudaError_t boundary_configure_batched(const size_t *smem) {
-    cudaError_t e;
-    e = cudaFuncSetAttribute(k_rows_fwd_b<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem[0]);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_cols_b<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem[1]);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_rows_inv_b<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem[2]);
+    cudaError_t e = allow_shared(k_rows_fwd_b<T>, smem[0]);
+    if (e == cudaSuccess) e = allow_shared(k_cols_b<T>, smem[1]);
+    if (e == cudaSuccess) e = allow_shared(k_rows_inv_b<T>, smem[2]);
     return e;
 }
 

@@ -19,6 +19,20 @@
 
 namespace tcsem {
 
+// The limit on a kernel's dynamic shared memory belongs to the function, not to the handle that sets it: every
+// handle sets the most a block may have, so that none lowers another's.  An error where `need` is more.
+template <typename K> inline cudaError_t allow_shared(K *kernel, size_t need) {
+    int dev = 0, most = 0;
+    cudaFuncAttributes fa;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, kernel);
+    if (e != cudaSuccess) return e;
+    most -= (int)fa.sharedSizeBytes;
+    if (need > (size_t)most) return cudaErrorInvalidValue;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+}
+
 struct Geom {
     int L, M, N;
     int XP, YP;

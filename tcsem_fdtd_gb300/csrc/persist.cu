@@ -187,7 +187,7 @@ template <typename T> __global__ void k_queue_seed(const __grid_constant__ Persi
 }
 
 template <typename T> cudaError_t persist_configure(size_t smem) {
-    return cudaFuncSetAttribute(k_persistent<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    return allow_shared(k_persistent<T>, smem);
 }
 
 template <typename T> int persist_blocks(size_t smem) {

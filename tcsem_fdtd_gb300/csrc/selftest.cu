@@ -25,7 +25,7 @@ cudaError_t launch_sweep_lost(const SweepMaps &maps, const Geom &g, const T *tin
                               const SourceTable<T> &src, int rows, int *err, int *loaded, cudaStream_t st) {
     ZChunks zc{1, rows, {0, g.N}};
     const size_t sm = sweep_smem_bytes<T>(g.N);
-    cudaError_t e = cudaFuncSetAttribute(k_sweep_lost<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    const cudaError_t e = allow_shared(k_sweep_lost<T>, sm);
     if (e != cudaSuccess) return e;
     k_sweep_lost<T><<<dim3(sweep_tiles_x(g.L), sweep_tiles_y(g.M, rows)), fs3::NT, sm, st>>>(maps, g, tin, tout, ax, s, src,
                                                                                            zc, err, loaded);

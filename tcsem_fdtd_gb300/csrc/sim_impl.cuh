@@ -535,7 +535,7 @@ template <typename T> struct SimImpl : SimBase {
             int maxsm = 0;
             CK(cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
             if (st_smem > (size_t)maxsm) return false;
-            CK(steps_configure<T>(maxsm));  // the most for any grid: the limit is the function's, not the handle's
+            CK(steps_configure<T>(st_smem));
             const int slots = steps_blocks<T>(st_smem), tiles = sweep_tiles_x(m.L) * sweep_tiles_y(m.M, zc.rows);
             sa.nfwd = tiles_fwd(d);
             sa.ninv = tiles_inv(d);
@@ -1143,7 +1143,12 @@ template <typename T> struct SimImpl : SimBase {
         for (int s = 0; s < gsteps; s++) enqueue_step(b ^ (s & 1), StepGate{gate_base.as<int>(), s, sched.nsteps});
         rx_close();
         launch_advance(gate_base.as<int>(), gsteps, stream);
+        const cudaError_t refused = cudaGetLastError();  // of a launch: the graph lacks it
         cudaError_t e = cudaStreamEndCapture(stream, &graph);
+        if (e == cudaSuccess && refused != cudaSuccess) {
+            cudaGraphDestroy(graph);
+            e = refused;
+        }
         if (e != cudaSuccess) throw Error(TCSEM_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
         e = cudaGraphInstantiateWithFlags(&gexec[b], graph, cudaGraphInstantiateFlagUseNodePriority);
         cudaGraphDestroy(graph);

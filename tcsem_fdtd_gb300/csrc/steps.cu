@@ -175,7 +175,7 @@ template <typename T> size_t steps_smem(const Products<T> &d, int N) {
 }
 
 template <typename T> cudaError_t steps_configure(size_t smem) {
-    return cudaFuncSetAttribute(k_steps<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    return allow_shared(k_steps<T>, smem);
 }
 
 template <typename T> int steps_blocks(size_t smem) {

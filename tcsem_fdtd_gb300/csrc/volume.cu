@@ -202,11 +202,9 @@ int sweep_tiles_x(int L) { return (L + fs3::TX - 1) / fs3::TX; }
 int sweep_tiles_y(int M, int rows) { return (M + rows - 1) / rows; }
 
 template <typename T> cudaError_t sweep_configure(int N) {
-    const int sm = (int)fs3::smem_bytes_n<T>(N);
-    cudaError_t e = cudaFuncSetAttribute(k_sweep<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-    if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(k_sweep_batched<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                sm < (int)kAloneBytes ? (int)kAloneBytes : sm);
+    const size_t sm = fs3::smem_bytes_n<T>(N);
+    const cudaError_t e = allow_shared(k_sweep<T>, sm);
+    return e != cudaSuccess ? e : allow_shared(k_sweep_batched<T>, sm);
 }
 template <typename T> size_t sweep_smem_bytes(int N) { return fs3::smem_bytes_n<T>(N); }
 template <typename T> int sweep_blocks_per_sm(int N) {
