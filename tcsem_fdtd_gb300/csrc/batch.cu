@@ -181,14 +181,16 @@ template <typename T> struct BatchImpl : BatchBase {
         const int n = (int)running.size();
         bool whole = !persistent && n > 0;
         long tiles = 0;
+        int deepest = 1;
         for (int q : running) {
             const SimImpl<T> &m = *slots[q].sim;
+            deepest = std::max(deepest, m.g.N);
             whole = whole && m.zc.n == 1 && m.g.N >= 2;
             tiles += m.sweep_blocks();
         }
         int sms = 0;
         CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-        const long slots_sm = sizeof(T) == 4 ? 2 : 1;
+        const long slots_sm = sweep_blocks_per_sm<T>(deepest);
         pieces = whole && 10 * tiles <= 7 * slots_sm * sms;
         spread = pieces && 3 * tiles <= 2 * sms;
         ngroups = whole && !pieces && n > 1 ? 2 : 1;

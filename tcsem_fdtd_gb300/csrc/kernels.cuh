@@ -136,6 +136,7 @@ template <typename T> int sweep_blocks_per_sm(int N);  // resident sweep CTAs pe
 int sweep_box_x();
 int sweep_box_y();
 int sweep_tile_x();
+int sweep_table_planes();  // planes of a march beyond which its z table is filled again
 template <typename T> void launch_bz_consolidate(const Geom &g, T *bz, T *tot, const ZChunks &zc, cudaStream_t st);
 // nx x ny cells of planes k .. k+n-1 of a volume as dense doubles, and back
 template <typename T> void launch_crop(const Geom &g, const T *v, double *out, int nx, int ny, int k, int n, cudaStream_t st);

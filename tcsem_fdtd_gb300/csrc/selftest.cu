@@ -17,7 +17,7 @@ template <typename T>
 __global__ void __launch_bounds__(fs3::NT, sizeof(T) == 4 ? 2 : 1)
     k_sweep_lost(const __grid_constant__ SweepMaps maps, Geom g, const T *__restrict__ tin, T *__restrict__ tout, Axis<T> ax,
                  StepScalars<T> s, SourceTable<T> src, ZChunks zc, int *err, int *loaded) {
-    sweep_cta<T, false, 2>(maps, g, tin, tout, ax, s, src, zc, blockIdx.x, blockIdx.y, 0, err, NoPatience{loaded});
+    sweep_cta<T, false, 2, true>(maps, g, tin, tout, ax, s, src, zc, blockIdx.x, blockIdx.y, 0, err, NoPatience{loaded});
 }
 
 template <typename T>

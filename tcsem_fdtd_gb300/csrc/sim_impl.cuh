@@ -412,14 +412,21 @@ template <typename T> struct SimImpl : SimBase {
     }
 
     // z-chunk layout: n chunks, the top one `top` planes deep (top <= 0: an even split)
-    void set_chunks(int n, int top) {
+    ZChunks chunks(int n, int top) const {
         const int N = model.N;
-        zc.n = n;
-        for (int c = 0; c <= n; c++) zc.kb[c] = (int)(((long)c * N) / n);
+        ZChunks z{n, zc.rows, {}};
+        for (int c = 0; c <= n; c++) z.kb[c] = (int)(((long)c * N) / n);
         if (n > 1 && top > 0) {
             top = std::max(1, std::min(top, N - (n - 1)));
-            for (int c = 1; c <= n; c++) zc.kb[c] = top + (int)(((long)(c - 1) * (N - top)) / (n - 1));
+            for (int c = 1; c <= n; c++) z.kb[c] = top + (int)(((long)(c - 1) * (N - top)) / (n - 1));
         }
+        return z;
+    }
+    void set_chunks(int n, int top) { zc = chunks(n, top); }
+    static int deepest(const ZChunks &z) {
+        int d = 0;
+        for (int c = 0; c < z.n; c++) d = std::max(d, z.kb[c + 1] - z.kb[c]);
+        return d;
     }
     // most chunks a layout may have: every chunk keeps at least 8 planes
     int max_chunks() const { return std::max(1, std::min(kMaxChunks, model.N / 8)); }
@@ -433,7 +440,9 @@ template <typename T> struct SimImpl : SimBase {
         int sms = 0;
         CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
         CK(sweep_configure<T>(m.N));
-        const int per_sm = sweep_blocks_per_sm<T>(m.N);
+        // The layout decides the last bits of Bz and which saved states continue.  In FP32 it counts one CTA per SM from
+        // 967 planes on, where a table of all planes (12 bytes each, beside 104,080) once left room for one.
+        const int per_sm = sizeof(T) == 4 && m.N > 966 ? 1 : sweep_blocks_per_sm<T>(m.N);
         const long slots = (long)sms * per_sm;
         long tiles = (long)sweep_tiles_x(m.L) * sweep_tiles_y(m.M, zc.rows);
         int n, top = 0, most = max_chunks();
@@ -509,7 +518,7 @@ template <typename T> struct SimImpl : SimBase {
     void plan_steps() {
         if constexpr (sizeof(T) == 4) {
             const Model &m = model;
-            if (!steps_possible()) return;
+            if (!steps_possible() || deepest(zc) > sweep_table_planes()) return;  // its sweep fills no table twice
             const int L1 = bd.L1, M1 = bd.M1;
             Products<T> &d = sa.pd;
             products_shape(d, m.L, m.M, L1, M1, true);
@@ -706,13 +715,17 @@ template <typename T> struct SimImpl : SimBase {
             for (int b = 0; b < 2; b++) {
                 sa.maps[b] = maps[b];
                 sa.f[b] = fs(b);
-                sa.tot[b] = tot[b].as<T>();
             }
-            sa.g = g; sa.ax = ax; sa.table = steps.as<StepScalars<T>>(); sa.zc = zc;
+            bind_layout();
+            sa.g = g; sa.ax = ax; sa.table = steps.as<StepScalars<T>>();
             sa.ctl = st_ctl.as<int>();
             sa.err = errw.as<int>();
             sa.wait_ns = 2000000000LL;
         }
+    }
+    void bind_layout() {
+        for (int b = 0; b < 2; b++) sa.tot[b] = tot[b].as<T>();
+        sa.zc = zc;
     }
     void advance_steps(long todo) {
         if constexpr (sizeof(T) == 4) {
@@ -1416,13 +1429,19 @@ template <typename T> struct SimImpl : SimBase {
         ok = (std::fclose(f) == 0) && ok;
         if (!ok) throw Error(TCSEM_ERR_IO, std::string("cannot write ") + path);
     }
-    int earlier_chunks() const {
+    // The layouts that states of a handle with the default options may be in: today's default; in FP64 the one before
+    // tile heights and chunk counts were chosen together; in FP32, of grids of 230 to 966 planes, the one of a sweep
+    // that had one CTA on an SM there.
+    std::vector<ZChunks> default_layouts() const {
         int sms = 0;
         CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
         const long tiles = (long)sweep_tiles_x(model.L) * sweep_tiles_y(model.M, 8);
         long lower = std::max<long>(1, sms * 85L / 100 / tiles);
-        if ((lower + 1) * tiles <= sms) lower++;
-        return (int)std::min<long>(1 + lower, max_chunks());
+        if (sizeof(T) == 8 && (lower + 1) * tiles <= sms) lower++;
+        std::vector<ZChunks> v{chunks(1 + rule_lower, 1)};
+        if (sizeof(T) == 8 || (model.N >= 230 && model.N <= 966))
+            v.push_back(chunks((int)std::min<long>(1 + lower, max_chunks()), 1));
+        return v;
     }
     void adopt_layout(const ZChunks &lay) {
         CK(cudaStreamSynchronize(stream));
@@ -1433,9 +1452,10 @@ template <typename T> struct SimImpl : SimBase {
             dev_bytes += tb - tot[b].n;
             tot[b].alloc(tb);
         }
-        overlap = overlap && zc.n > 1;
+        overlap = side && zc.n > 1;
+        if (steps_on) bind_layout();
         chunks_used = zc.n;
-        top_used = overlap ? zc.kb[1] : 0;
+        top_used = zc.n > 1 && (overlap || steps_on) ? zc.kb[1] : 0;
     }
     // into a handle of the same survey, precision and z-chunk layout; the run continues with advance
     void load_state(const char *path) override {
@@ -1449,15 +1469,10 @@ template <typename T> struct SimImpl : SimBase {
             throw Error(st, m);
         };
         if (!ok || std::memcmp(h.magic, "TCSEMST", 8) != 0 || h.version != 2) fail(TCSEM_ERR_PARSE, std::string(path) + " is not a saved run state");
-        // a handle with the default layout also continues a state saved in the layout that was the default before
-        // the tile heights and chunk counts were chosen together
         ZChunks lay = zc;
-        if (sizeof(T) == 8 && ok && opts.zchunks == 0 && opts.top_planes == 0 && !opts.serial_boundary && h.nch != zc.n) {
-            const ZChunks now = zc;
-            set_chunks(earlier_chunks(), 1);
-            lay = zc;
-            zc = now;
-        }
+        if (opts.zchunks == 0 && opts.top_planes == 0 && !opts.serial_boundary)
+            for (const ZChunks &z : default_layouts())
+                if (z.n == h.nch && (!steps_on || deepest(z) <= sweep_table_planes())) lay = z;
         bool same = h.tsize == (int)sizeof(T) && h.L == model.L && h.M == model.M && h.N == model.N && h.nch == lay.n &&
                     h.field_bytes == (long long)fld[0][0].n && h.tot_bytes == (long long)lay.n * g.PS * (long long)sizeof(T) &&
                     (h.cur == 0 || h.cur == 1) && h.step >= 0 && h.step <= sched.nsteps && h.itx >= 0 &&

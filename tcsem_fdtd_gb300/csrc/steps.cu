@@ -115,7 +115,7 @@ __global__ void __launch_bounds__(fs3::NT, 2) k_steps(const __grid_constant__ St
             for (int c = r < a.march ? r + 1 : a.zc.n;; c += a.march) {
                 const bool top = c >= a.zc.n;
                 if (top && r != a.march - 1 + a.own) break;
-                const bool ok = sweep_cta<T, true>(a.maps[b], a.g, a.tot[b], a.tot[b ^ 1], a.ax, a.table[a.step0 + s], a.src,
+                const bool ok = sweep_cta<T, true, fs3::ring<T>(), false>(a.maps[b], a.g, a.tot[b], a.tot[b ^ 1], a.ax, a.table[a.step0 + s], a.src,
                                                    a.zc, tile % a.tiles_x, tile / a.tiles_x, top ? 0 : c, a.err,
                                                    AirFlag<T>{sy, (s + 1) * a.nbnd});
                 if (!ok) return sy.give_up();

@@ -62,12 +62,24 @@ enum { SEX = 0, SEY, SBZ };
 constexpr int kLost = 1 << 30;  // above every plane's number
 template <typename T> __host__ __device__ constexpr int xoff(int a, int q) { return ring<T>() * NARR * boxs<T>() + (2 * a + q) * XBUF; }
 template <typename T> __host__ __device__ constexpr int soff(int a, int q) { return xoff<T>(3, 0) + (3 * q + a) * SBUF; }
-// byte offset of the ring's mbarriers and the source planes; then the z tables
+// What the z table is made from: its values dtb/dz, 1/(dz[k-1]+dz[k]) and dz of a plane, the first two times a factor
+template <typename T> struct ZSource {
+    const T *rdz, *rdzs, *dzk;
+    T dtb, cf;
+};
+// byte offset of the ring's mbarriers, the source planes and the z table's source; then the z table
 template <typename T> __host__ __device__ constexpr size_t bars_offset() { return (size_t)soff<T>(0, 2) * sizeof(T); }
-template <typename T> __host__ __device__ constexpr size_t smem_bytes() { return bars_offset<T>() + ring<T>() * 8 + 16; }
-template <typename T> size_t smem_bytes_n(int N) {  // plus the z tables
-    return smem_bytes<T>() + 3 * (size_t)(N + 3) * 2 * sizeof(T);
+template <typename T> __host__ __device__ constexpr size_t zsource_offset() { return bars_offset<T>() + ring<T>() * 8 + 16; }
+template <typename T> __host__ __device__ constexpr size_t smem_bytes() { return zsource_offset<T>() + (sizeof(ZSource<T>) + 15) / 16 * 16; }
+// Planes of the z table.  A deeper march fills it again on its way (two barriers every 220 planes), so that two CTAs
+// share an SM in FP32 whatever the depth of the grid: with a table of all planes, each value twice, it was one
+// CTA from 230 planes on.
+constexpr int ZWIN = 224;
+template <typename T> size_t smem_bytes_n(int N) {  // plus the z table
+    return smem_bytes<T>() + 3 * (size_t)(N + 3 < ZWIN ? N + 3 : ZWIN) * 2 * sizeof(T);
 }
+// 228 KB of an SM, of which each CTA takes one more
+static_assert(2 * (smem_bytes<float>() + 3 * (size_t)ZWIN * 2 * sizeof(float) + 1024) <= (228 << 10), "two CTAs per SM in FP32");
 // the chunk offsets of Bz over the box, for the planes below k1 and for k1 itself, lie in the first
 // buffers of the stored planes: they are in registers before the third plane of the march writes there
 static_assert(2 * BOX <= 3 * SBUF, "the offset boxes fit the first store buffers");
@@ -97,7 +109,7 @@ template <typename T> struct SweepThread {
     uint64_t *bars;
     int *s_src;  // first and last plane with a source segment in the tile
     const SweepMaps *maps;
-    int j, N, k0, k1, klow, ktop, i0, j0;
+    int j, N, k0, klow, ktop, i0, j0;  // planes k0 .. ktop - 1; klow: first plane of the z table
     int kend;     // last plane whose stage the thread waits for, or loads: k0, or kLost + the stage at which it gave up
     int role;     // 0: a row of the tile, 1: the +y halo row, 2: the +x halo column, 3: none (warp-uniform)
     int duty;     // 1: the thread issues the loads (a lane of warp 8), 2: the stores (of the +x warp)
@@ -326,7 +338,7 @@ __device__ __forceinline__ void sweep_plane(SweepThread<T> &t, int k, int slot, 
             if constexpr (KIND == INNER || KIND == LAST) {
                 tma_store_3d(t.maps->o + 3, sm + xoff<T>(XBX, QB), t.i0, t.j0, k + 1);
                 tma_store_3d(t.maps->o + 4, sm + xoff<T>(XBY, QB), t.i0, t.j0, k + 1);
-                if (k + 2 < t.k1) tma_store_3d(t.maps->o + 5, sm + soff<T>(SBZ, QB), t.i0, t.j0, k + 2);
+                if (k + 2 < t.ktop) tma_store_3d(t.maps->o + 5, sm + soff<T>(SBZ, QB), t.i0, t.j0, k + 2);
             }
             bulk_commit();
         } else if (KIND != LAST && k - RING >= t.kend) {  // the slot takes the stage RING planes up
@@ -353,12 +365,33 @@ template <typename T> __device__ __forceinline__ void set_offsets(SweepThread<T>
     }
 }
 
+// all threads: the z table for the planes klow ..., as far as it goes or the march needs
+template <typename T> __device__ __forceinline__ void fill_z(Pair<T> *s_z, const fs3::ZSource<T> &z, int klow, int ktop, int N) {
+    const int n = min(fs3::ZWIN, ktop + 2 - klow);
+    for (int e = threadIdx.x; e < n; e += fs3::NT) {
+        const int k = klow + e;
+        const bool in = k >= 0 && k < N;
+        s_z[3 * e] = dup<T>(in ? z.rdz[k] * z.dtb : T(0));
+        s_z[3 * e + 1] = dup<T>(in ? z.rdzs[k] * z.cf : T(0));
+        s_z[3 * e + 2] = dup<T>(in ? z.dzk[k] : T(0));
+    }
+}
+// all threads, between two planes: the table for the planes below k, down to k0 - 1 if they fit
+template <typename T> __device__ __forceinline__ void refill_z(SweepThread<T> &t, Pair<T> *s_z, int k) {
+    const fs3::ZSource<T> &z = *reinterpret_cast<const fs3::ZSource<T> *>(reinterpret_cast<const unsigned char *>(t.sm) + fs3::zsource_offset<T>());
+    __syncthreads();  // the last plane's readers are done
+    t.klow = max(t.k0 - 1, k + 1 - fs3::ZWIN);
+    fill_z(s_z, z, t.klow, k - 1, t.N);
+    __syncthreads();
+}
+
 // The z-march of one warp through the chunk, in the copy of the plane code for its role.  COPIES of the inner plane:
 // RING with the slots as constants, or 2 with the slot in a register and half of the code (256 x 256 x 160
 // 131.2 -> 128.7 us per step, in FP64 1348 -> 1336).  The batched and the cooperative kernel keep RING in FP32: there the
 // register is one too many (8 surveys of up to 152 x 131 x 112 170 -> 174 us, 64 x 64 x 48 19.2 -> 19.3).
-template <typename T, int ROLE, int COPIES, typename Air>
-__device__ __forceinline__ void sweep_march(SweepThread<T> &t, const StepScalars<T> &s, const Pair<T> *s_z,
+// DEEP: the march may have more planes than the z table.
+template <typename T, int ROLE, int COPIES, bool DEEP, typename Air>
+__device__ __forceinline__ void sweep_march(SweepThread<T> &t, const StepScalars<T> &s, Pair<T> *s_z,
                                             const SourceTable<T> &src, const T *s_oc, const Air &air) {
     using namespace fs3;
     constexpr int RING = ring<T>();
@@ -371,7 +404,9 @@ __device__ __forceinline__ void sweep_march(SweepThread<T> &t, const StepScalars
     sweep_plane<T, 1, SECOND, ROLE>(t, k, 1 % RING, 1 / RING, s, s_z, src, air);
     if constexpr (COPIES == 2) {
         int n = 2;  // planes done
-        while (--k >= k0) {
+        for (;;) {
+            if (DEEP && t.klow >= k0 && k - 2 < t.klow) refill_z(t, s_z, k);
+            if (--k < k0) break;
             sweep_plane<T, 0, INNER, ROLE>(t, k, n % RING, n / RING, s, s_z, src, air);
             n++;
             if (--k < k0) break;
@@ -382,7 +417,9 @@ __device__ __forceinline__ void sweep_march(SweepThread<T> &t, const StepScalars
         else sweep_plane<T, 0, LAST, ROLE>(t, k, n % RING, n / RING, s, s_z, src, air);
     } else {
         int round = 0, left = 2;  // slot of the plane after the last inner one
-        while (--k >= k0) {
+        for (;;) {
+            if (DEEP && t.klow >= k0 && k - 4 < t.klow) refill_z(t, s_z, k);
+            if (--k < k0) break;
             sweep_plane<T, 0, INNER, ROLE>(t, k, 2, round, s, s_z, src, air);
             if (--k < k0) { left = 3; break; }
             sweep_plane<T, 1, INNER, ROLE>(t, k, 3, round, s, s_z, src, air);
@@ -402,7 +439,7 @@ __device__ __forceinline__ void sweep_march(SweepThread<T> &t, const StepScalars
 // one CTA of the sweep: tile (bx, by) of z-chunk c (or a piece of the only chunk) with the step scalars s.  FRESH: the chunk
 // totals tin may have been written by another CTA of the same launch (persistent schedule).  False (for all threads): a
 // copy did not arrive; it is recorded in err, and no copy is in flight.
-template <typename T, bool FRESH = false, int COPIES = fs3::ring<T>(), typename Air = AirAfterKernel>
+template <typename T, bool FRESH = false, int COPIES = fs3::ring<T>(), bool DEEP = true, typename Air = AirAfterKernel>
 __device__ __forceinline__ bool sweep_cta(const SweepMaps &maps, const Geom &g, const T *__restrict__ tin,
                                           T *__restrict__ tout, const Axis<T> &ax, StepScalars<T> s,
                                           const SourceTable<T> &src, const ZChunks &zc, int bx, int by, int c, int *err,
@@ -418,7 +455,7 @@ __device__ __forceinline__ bool sweep_cta(const SweepMaps &maps, const Geom &g, 
     t.bars = reinterpret_cast<uint64_t *>(smem_raw + bars_offset<T>());
     static_assert(bars_offset<T>() % 128 == 0, "the new planes are whole 128-byte lines");
     t.s_src = reinterpret_cast<int *>(t.bars + RING);
-    Pair<T> *s_z = reinterpret_cast<Pair<T> *>(smem_raw + smem_bytes<T>());  // [N+3][3], each value twice
+    Pair<T> *s_z = reinterpret_cast<Pair<T> *>(smem_raw + smem_bytes<T>());  // [ZWIN][3] at most, each value twice
     t.maps = &maps;
 
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
@@ -427,7 +464,7 @@ __device__ __forceinline__ bool sweep_cta(const SweepMaps &maps, const Geom &g, 
     const int L = g.L, M = g.M, N = g.N, XP = g.XP, PS = (int)g.PS;
     t.N = N;
     t.k0 = zc.plane(c) + (piece == Piece::LOWER ? 1 : 0);
-    t.k1 = piece == Piece::TOP ? t.k0 + 1 : zc.plane(c + 1);
+    t.ktop = piece == Piece::TOP ? t.k0 + 1 : zc.plane(c + 1);  // first plane of the march: the halo plane of the chunk below, or the zero bottom
     // rows: cells x = lane, lane + 32 of row w; column warp: one cell per lane, x = 64 of row `lane`.  A tile
     // has zc.rows rows, warp zc.rows computes the halo row and the warps between it and the column's idle.
     const bool column = w == 9;
@@ -465,16 +502,11 @@ __device__ __forceinline__ bool sweep_cta(const SweepMaps &maps, const Geom &g, 
     t.rdx2 = pair<T>(r2[0], r2[1]);
     t.rdx = pair<T>(r1[0], r1[1]);
     t.fx = pair<T>(r1[0] * s.dtb, r1[1] * s.dtb);
-    t.ktop = t.k1 < N ? t.k1 : N;  // first plane: the chunk's halo plane below, or the zero bottom
-    t.klow = t.k0 - 1;
-    const int ktop = t.ktop, klow = t.klow;
-    for (int e = tid; e <= ktop + 1 - klow; e += NT) {
-        const int k = klow + e;
-        const bool in = k >= 0 && k < N;
-        s_z[3 * e] = dup<T>(in ? ax.rdz[k] * s.dtb : T(0));
-        s_z[3 * e + 1] = dup<T>(in ? ax.rdzs[k] * cf : T(0));
-        s_z[3 * e + 2] = dup<T>(in ? ax.dzk[k] : T(0));
-    }
+    const int ktop = t.ktop;
+    t.klow = DEEP ? max(t.k0 - 1, ktop + 2 - ZWIN) : t.k0 - 1;  // entries of planes ktop and ktop + 1 among them
+    const ZSource<T> zsrc{ax.rdz, ax.rdzs, ax.dzk, s.dtb, cf};
+    fill_z(s_z, zsrc, t.klow, ktop, N);
+    if (DEEP && tid == 0) *reinterpret_cast<ZSource<T> *>(smem_raw + zsource_offset<T>()) = zsrc;
 
     bool src_tile = false;  // tile-uniform: does any source segment touch this tile, and on which planes?
     int sk0 = N, sk1 = -1;
@@ -531,7 +563,7 @@ __device__ __forceinline__ bool sweep_cta(const SweepMaps &maps, const Geom &g, 
     t.ex1 = t.ey1 = t.exn = t.eyn = t.ezn = dup<T>(T(0));
     t.bxo1 = t.byo1 = t.bxn = t.byn = t.acc = dup<T>(T(0));
     if (piece == Piece::TOP && t.role == 0 && t.j < M) {  // the sum up to the plane below
-        const long long o = g.at(t.i, t.j, t.k1);
+        const long long o = g.at(t.i, t.j, t.ktop);
         if (t.i < L && TCSEM_IN(o, g.total(), err)) t.acc.a = __ldcg(bz_new + o);
         if (t.i + 32 < L && TCSEM_IN(o + 32, g.total(), err)) t.acc.b = __ldcg(bz_new + o + 32);
     }
@@ -547,18 +579,18 @@ __device__ __forceinline__ bool sweep_cta(const SweepMaps &maps, const Geom &g, 
     // (5 % faster).  FP32 runs one copy in every warp: three copies of its loop made the sweep 40 %
     // slower (measured; presumably the larger loop no longer fits the instruction cache).
     if constexpr (sizeof(T) == 8) {
-        if (t.role == 0) sweep_march<T, 0, COPIES>(t, s, s_z, src, s_oc, air);
-        else if (t.role == 1) sweep_march<T, 1, COPIES>(t, s, s_z, src, s_oc, air);
-        else if (t.role == 2) sweep_march<T, 2, COPIES>(t, s, s_z, src, s_oc, air);
-        else sweep_march<T, 3, COPIES>(t, s, s_z, src, s_oc, air);
+        if (t.role == 0) sweep_march<T, 0, COPIES, DEEP>(t, s, s_z, src, s_oc, air);
+        else if (t.role == 1) sweep_march<T, 1, COPIES, DEEP>(t, s, s_z, src, s_oc, air);
+        else if (t.role == 2) sweep_march<T, 2, COPIES, DEEP>(t, s, s_z, src, s_oc, air);
+        else sweep_march<T, 3, COPIES, DEEP>(t, s, s_z, src, s_oc, air);
     } else {
-        sweep_march<T, 0, COPIES>(t, s, s_z, src, s_oc, air);
+        sweep_march<T, 0, COPIES, DEEP>(t, s, s_z, src, s_oc, air);
     }
     // the last plane's Bz, in the buffer of its parity
     async_shared_fence();
     const bool bad = __syncthreads_or(t.kend >= kLost);
     if (t.duty == 2) {
-        tma_store_3d(maps.o + 5, t.sm + ((ktop - klow) & 1 ? soff<T>(SBZ, 1) : soff<T>(SBZ, 0)), t.i0, t.j0, t.k0);
+        tma_store_3d(maps.o + 5, t.sm + ((ktop - t.k0) & 1 ? soff<T>(SBZ, 0) : soff<T>(SBZ, 1)), t.i0, t.j0, t.k0);
         bulk_commit();
         bulk_wait_all();
     }

@@ -216,6 +216,7 @@ template <typename T> int sweep_blocks_per_sm(int N) {
 int sweep_box_x() { return fs3::BXW; }
 int sweep_box_y() { return fs3::BYH; }
 int sweep_tile_x() { return fs3::TX; }
+int sweep_table_planes() { return fs3::ZWIN - 3; }
 
 // Materialise Bz = P + O_c in place; the caller clears the chunk totals.  Bound by latency on the grids that a host
 // steps stage by stage: one thread per column and chunk, eight planes in flight (64 x 64 x 48 with six chunks:
