@@ -369,10 +369,10 @@ template <typename T> struct SimImpl : SimBase {
     }
 
     // The layout autotuner (tcsem_opts.zchunks = -1): times a captured block of 8 steps for
-    // each layout near the rule of init_chunks -- one to five lower chunks around it, a
-    // one-plane or an even top chunk -- and keeps the fastest.  The Bz prefix is summed per
-    // chunk, so the layout decides the order of some FP additions: with the tuner the last
-    // bits may differ between runs whose timings chose differently.
+    // each layout near the rule of init_chunks -- one to five lower chunks around it (the rule's own
+    // count among them), a one-plane or an even top chunk -- and keeps the fastest.  The tile height stays the rule's.
+    // The Bz prefix is summed per chunk, so the layout decides the order of some FP additions: with the tuner
+    // the last bits may differ between runs whose timings chose differently.
     int rule_lower = 1;  // lower chunks the rule of init_chunks chose
     void tune_layout() {
         if (itx < 0) select(0);
@@ -381,7 +381,7 @@ template <typename T> struct SimImpl : SimBase {
         CK(cudaEventCreate(&e1));
         struct Cand { int n, top; };
         std::vector<Cand> cands;
-        for (int lower = std::max(1, rule_lower - 2); lower <= rule_lower + 2 && lower + 1 <= max_chunks(); lower++)
+        for (int lower = std::max(1, rule_lower - 2); lower <= rule_lower + 2 && lower < rule_chunks() && deep_enough(lower); lower++)
             for (int top : {1, 0}) cands.push_back({lower + 1, top});
         const int keep = gsteps;
         gsteps = 8;
@@ -430,6 +430,10 @@ template <typename T> struct SimImpl : SimBase {
     }
     // most chunks a layout may have: every chunk keeps at least 8 planes
     int max_chunks() const { return std::max(1, std::min(kMaxChunks, model.N / 8)); }
+    // ... of the rule of init_chunks and the autotuner's candidates: in FP64, beside the boundary, any number of lower
+    // chunks of at least two planes
+    int rule_chunks() const { return sizeof(T) == 8 && !opts.serial_boundary ? kMaxChunks : max_chunks(); }
+    bool deep_enough(int lower) const { return sizeof(T) == 4 || lower == 1 || (model.N - 1) / lower >= 2; }
     // z-chunks (and FP64: tile rows) of the fused sweep.  Overlapped step: a one-plane top chunk (the only part of
     // the sweep that waits for the boundary) and lower chunks whose CTAs fit in one wave;
     // deeper chunks also mean fewer halo planes.  In FP32 the sweep is bound by memory and
@@ -445,7 +449,7 @@ template <typename T> struct SimImpl : SimBase {
         const int per_sm = sizeof(T) == 4 && m.N > 966 ? 1 : sweep_blocks_per_sm<T>(m.N);
         const long slots = (long)sms * per_sm;
         long tiles = (long)sweep_tiles_x(m.L) * sweep_tiles_y(m.M, zc.rows);
-        int n, top = 0, most = max_chunks();
+        int n, top = 0;
         if (opts.serial_boundary) {
             n = (int)std::min<long>(kMaxChunks, std::max<long>(1, (7L * sms + tiles - 1) / tiles));
         } else if (sizeof(T) == 8) {
@@ -462,7 +466,7 @@ template <typename T> struct SimImpl : SimBase {
             int lower = 1;
             for (int r = 8; r >= 3; r--) {
                 const long tl = (long)sweep_tiles_x(m.L) * sweep_tiles_y(m.M, r);
-                for (int q = 1; q < kMaxChunks && (q == 1 || (m.N - 1) / q >= 2); q++) {
+                for (int q = 1; q < kMaxChunks && deep_enough(q); q++) {
                     const long waves = (tl * q + slots - 1) / slots, left = slots - tl * q;
                     const double low = 4 + waves * 0.95 * (r + 1) * ((m.N - 1 + q - 1) / q + 1.25),
                                  last = 4 + 0.95 * (r + 1) * 3 * ((tl + slots - 1) / slots),
@@ -474,18 +478,17 @@ template <typename T> struct SimImpl : SimBase {
             if (opts.zchunks > 0) zc.rows = 8;
             n = 1 + lower;
             top = 1;
-            most = kMaxChunks;
         } else {
             n = 1 + (int)std::max<long>(1, slots * 85 / 100 / tiles);
             top = 1;
         }
-        n = std::min(n, most);
+        n = std::min(n, rule_chunks());
         rule_lower = n - 1;
         if (opts.zchunks > 0) n = std::min(std::min(opts.zchunks, kMaxChunks), m.N);
         if (opts.top_planes != 0) top = opts.top_planes;  // > 0: that many planes, < 0: an even split
         set_chunks(n, top);
         // the autotuner may pick up to two more lower chunks than the rule
-        int nalloc = opts.zchunks < 0 ? std::max(n, std::min(rule_lower + 3, max_chunks())) : n;
+        int nalloc = opts.zchunks < 0 ? std::max(n, std::min(rule_lower + 3, rule_chunks())) : n;
         nalloc = std::max(nalloc, std::min(tot_chunks_min, max_chunks()));
         const size_t tb = (size_t)nalloc * g.PS * sizeof(T);
         for (int b = 0; b < 2; b++) {
