@@ -93,7 +93,8 @@ __device__ __forceinline__ float rcp_fast(float x) {
 }
 // In FP64 the hardware's approximation r0 of 1/x (a MUFU op, about 20 bits) and one third-order step of
 // Householder's iteration, 1/x = r0 / (1 - e) = r0 (1 + e + e^2 + ...) with e = 1 - x r0: what is left out is
-// e^3 ~ 2^-60, and three FP64 operations take the place of a division's (normal x only)
+// e^3, and three FP64 operations take the place of a division's.  For normal x with a normal reciprocal: here
+// x = 2 gamma + sigma dt with gamma > 0.  IEEE division's result or a neighbour of it (tests/test_gpu_reciprocal.py).
 __device__ __forceinline__ double rcp64(double x) {
     double r;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
