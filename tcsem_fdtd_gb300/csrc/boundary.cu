@@ -87,11 +87,21 @@ __global__ void k_bilinear_b(const BoundarySlot<T> *__restrict__ slots, const __
 }
 
 template <typename T> static size_t smem_rows(const BoundaryDev<T> &bd, int L) { return rows_fwd_layout(bd, L).total; }
-template <typename T> static size_t smem_cols(const BoundaryDev<T> &bd) {
-    const size_t t = cols_layout(bd).total;
-    return t > bd.cols_pad ? t : bd.cols_pad;
-}
+template <typename T> static size_t smem_cols(const BoundaryDev<T> &bd) { return cols_layout(bd).total; }
 template <typename T> size_t cols_apart(const BoundaryDev<T> &bd) { return cols_layout(bd).apart; }
+// The columns' blocks start while the row stage's still hold some SMs, and crowd on the others.  Alone, 369 blocks of a
+// 736 x 736 plane (35 KB each) in FP32: 47 or 37 us for the whole boundary from one process to the next, 35.4 with at most
+// three on an SM; in FP64 160.  No region on top of another (55 and 110 KB): 36 to 39, and 170.
+template <typename T> size_t cols_even(const BoundaryDev<T> &bd) {
+    int dev = 0, sms = 0, sm = 0, most = 0, own = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&own, cudaDevAttrReservedSharedMemoryPerBlock, dev) != cudaSuccess)
+        return 0;
+    const int share = (bd.H + sms - 1) / sms, bytes = sm / share - own;
+    return share == 1 || bytes <= 0 ? 0 : (size_t)(bytes < most ? bytes : most) / 128 * 128;
+}
 template <typename T> static size_t smem_inv(const BoundaryDev<T> &bd) { return rows_inv_layout(bd).total; }
 
 template <typename T> size_t boundary_smem_need(const BoundaryDev<T> &bd, int L) {
@@ -101,7 +111,7 @@ template <typename T> size_t boundary_smem_need(const BoundaryDev<T> &bd, int L)
 
 template <typename T> cudaError_t boundary_configure(const BoundaryDev<T> &bd, int L) {
     cudaError_t e = allow_shared(k_rows_fwd<T>, smem_rows(bd, L));
-    if (e == cudaSuccess) e = allow_shared(k_cols<T>, cols_apart(bd));
+    if (e == cudaSuccess) e = allow_shared(k_cols<T>, cols_layout(bd).apart);
     if (e == cudaSuccess) e = allow_shared(k_rows_inv<T>, smem_inv(bd));
     return e;
 }
@@ -154,12 +164,13 @@ cudaError_t launch_boundary_batched(const BoundarySlot<T> *slots, const BatchInd
 
 template <typename T>
 void launch_boundary(const BoundaryDev<T> &bd, const Geom &g, const T *bz, const T *tot, int nch, T *bx, T *by,
-                     StepGate gate, cudaStream_t st, bool pdl) {
+                     StepGate gate, cudaStream_t st, size_t cols_smem, bool pdl) {
     k_rows_fwd<T><<<(g.M + 1) / 2, kBndThreads, smem_rows(bd, g.L), st>>>(bd, bz, tot, nch, g, gate);
     // The column stage starts early only where the caller asks (beside a long sweep its early CTAs
     // would take slots the sweep's single wave needs at the start of a step); the last two stages
     // always do: by then the sweep's CTAs are all resident.
-    launch_after(pdl, k_cols<T>, bd.H, kBndThreads, smem_cols(bd), st, bd, gate);
+    const size_t cols = smem_cols(bd) > cols_smem ? smem_cols(bd) : cols_smem;
+    launch_after(pdl, k_cols<T>, bd.H, kBndThreads, cols, st, bd, gate);
     launch_after(true, k_rows_inv<T>, bd.S, kBndThreads, smem_inv(bd), st, bd, gate);
     int n = (g.L + 1) * g.M + g.L * (g.M + 1);
     launch_after(true, k_bilinear<T>, (n + 255) / 256, 256, (size_t)0, st, bd, bx, by, g, gate);
@@ -167,10 +178,11 @@ void launch_boundary(const BoundaryDev<T> &bd, const Geom &g, const T *bz, const
 
 #define INST(T)                                                                                            \
     template size_t cols_apart<T>(const BoundaryDev<T> &);                                                        \
+    template size_t cols_even<T>(const BoundaryDev<T> &);                                                         \
     template size_t boundary_smem_need<T>(const BoundaryDev<T> &, int);                                   \
     template cudaError_t boundary_configure<T>(const BoundaryDev<T> &, int);                              \
     template void launch_boundary<T>(const BoundaryDev<T> &, const Geom &, const T *, const T *, int, T *, T *,  \
-                                     StepGate, cudaStream_t, bool);                                       \
+                                     StepGate, cudaStream_t, size_t, bool);                                     \
     template BoundaryBlocks boundary_blocks<T>(const BoundaryDev<T> &, const Geom &);                     \
     template cudaError_t launch_boundary_batched<T>(const BoundarySlot<T> *, const BatchIndex *, const size_t *, int, \
                                                     cudaStream_t);                                        \

@@ -33,7 +33,6 @@ template <typename T> struct AxisRemap {
 };
 
 template <typename T> struct BoundaryDev {
-    size_t cols_pad = 0;  // shared memory that a block of the column stage asks for at least
     // plane geometry: the transforms have L1 x M1 points; the uniform grid (Lu x Mu points)
     // sits at offset (DL, DM) in them.  Without padding Lu = L1, Mu = M1, DL = DM = 0; with
     // padding the points outside the grid taper each row (column) from its edge values to
@@ -82,13 +81,17 @@ struct BoundaryBlocks {
 
 namespace tcsem {
 template <typename T> size_t boundary_smem_need(const BoundaryDev<T> &bd, int L);
-template <typename T> size_t cols_apart(const BoundaryDev<T> &bd);  // of the column stage with no region on top of another
+// Shared memory for a block of the column stage to ask for, beyond its need, so that the blocks do not crowd on few SMs:
+// as much as with no region on top of another, and so much that no SM takes more blocks than an even share (0 where that
+// is one block).
+template <typename T> size_t cols_apart(const BoundaryDev<T> &bd);
+template <typename T> size_t cols_even(const BoundaryDev<T> &bd);
 template <typename T> cudaError_t boundary_configure(const BoundaryDev<T> &bd, int L);
-// pdl: the last three kernels may start while their predecessor finishes (programmatic
+// cols_smem: shared memory that a block of the column stage asks for at least.  pdl: the last three kernels may start while their predecessor finishes (programmatic
 // dependent launch); off where the chain runs beside a long sweep whose CTAs need the slots
 template <typename T>
 void launch_boundary(const BoundaryDev<T> &bd, const Geom &g, const T *bz, const T *tot, int nch, T *bx, T *by,
-                     StepGate gate, cudaStream_t st, bool pdl = true);
+                     StepGate gate, cudaStream_t st, size_t cols_smem, bool pdl = true);
 template <typename T> BoundaryBlocks boundary_blocks(const BoundaryDev<T> &bd, const Geom &g);
 // idx[4] and smem[3]: the block lists of rows_fwd, cols, rows_inv, bilinear and the largest shared memory
 template <typename T>

@@ -189,6 +189,7 @@ template <typename T> struct SimImpl : SimBase {
     DevMem twx, twy, remT[2], remI[2], Gx, Gy, rows, FT, VX, VY, Zs, padx, pady;
     DevMem bxc_II, bxr_a, bxr_b, byc_II, byr_a, byr_b, bxc_l, bxr_l, byc_l, byr_l;
     BoundaryDev<T> bd{};
+    size_t cols_alone = 0, cols_beside = 0;  // shared memory of a column block without and beside a sweep (at least)
     // step tables
     DevMem steps, acts, gate_base;
     // transmitter dependent
@@ -355,16 +356,19 @@ template <typename T> struct SimImpl : SimBase {
         const float t_sweep = timed([&] { sweep(0, s, nullptr, StepGate{nullptr, 0, 0}); });
         const float t_bnd = timed([&] {
             FieldSet<T> f = fs(0);
-            launch_boundary<T>(bd, g, f.bz, tot[0].as<T>(), zc.n, f.bx, f.by, StepGate{nullptr, 0, 0}, stream, false);
+            launch_boundary<T>(bd, g, f.bz, tot[0].as<T>(), zc.n, f.bx, f.by, StepGate{nullptr, 0, 0}, stream, cols_alone, false);
         });
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
         CK(cudaGetLastError());
         overlap_pdl = t_bnd >= 0.5f * t_sweep;
-        // Where the boundary takes much longer than the sweep, its column blocks must not crowd on the SMs that the
-        // sweep leaves at first: two per SM there, and the rest everywhere once the sweep is done (247 x 117 x 49 with
-        // a 687 x 557 plane, the boundary 110 us and the sweep 21: 175 us per step with three, 156 with two).
-        if (t_bnd > 1.5f * t_sweep) bd.cols_pad = cols_apart(bd);
+        // Where the boundary takes longer than the sweep, its column blocks should not crowd on the SMs that the sweep
+        // leaves at first: fewer there, and the rest everywhere once the sweep is done.  us per step without and with
+        // larger blocks, by the ratio of the two times: 0.35 (256 x 256 x 160) 126.5 and 129.1, 0.8 (210 x 170 x 80) 58.5 and
+        // 60.5; 1.1 (three grids) 52.4, 61.0, 66.7 and 51.7, 59.5, 65.5; 1.3 (four) 53.2, 72.1, 49.8, 65.8 and 50.4, 65.4, 52.1, 68.7;
+        // 1.4 (180 x 180 x 60) 59.8 and 57.0; 1.6 (128 x 160 x 110) 69.8 and 73.0; 1.8 to 2.2 (five) 56.5, 66.3, 81.0, 77.1, 116.9 and
+        // 52.8, 62.7, 70.5, 70.4, 95.2; 2.9 97.2 and 92.3; 5.9 142.7 and 133.  Planes of up to 430 points: no difference.
+        if (t_bnd > t_sweep) cols_beside = cols_apart(bd);
         zero_state();
     }
 
@@ -1023,6 +1027,7 @@ template <typename T> struct SimImpl : SimBase {
             throw Error(TCSEM_ERR_INVALID, "continuation plane too large for the shared-memory FFT (" +
                                                std::to_string(L1) + " x " + std::to_string(M1) + ")");
         CK(boundary_configure(B, m.L));
+        cols_alone = cols_even(B);
     }
 
     void init_steps() {
@@ -1131,7 +1136,7 @@ template <typename T> struct SimImpl : SimBase {
         if (overlap) {  // fork: boundary -> top chunk on `side`; chunks 1.., then the previous step's receivers, on `stream`
             CK(cudaEventRecord(ev_fork, stream));
             CK(cudaStreamWaitEvent(side, ev_fork, 0));
-            launch_boundary<T>(bd, g, in.bz, tot[b].as<T>(), zc.n, in.bx, in.by, gate, side, overlap_pdl);
+            launch_boundary<T>(bd, g, in.bz, tot[b].as<T>(), zc.n, in.bx, in.by, gate, side, cols_beside, overlap_pdl);
             // the top chunk directly after the boundary's last stage, launched early: it stages its planes
             // while the bilinear remap runs and waits for it only before the air plane
             sweep(b, StepScalars<T>{}, table, gate, 0, 1, side, true);
@@ -1145,7 +1150,7 @@ template <typename T> struct SimImpl : SimBase {
             rx_gate = gate;
             return;
         } else {
-            launch_boundary<T>(bd, g, in.bz, tot[b].as<T>(), zc.n, in.bx, in.by, gate, stream);
+            launch_boundary<T>(bd, g, in.bz, tot[b].as<T>(), zc.n, in.bx, in.by, gate, stream, cols_alone);
             sweep(b, StepScalars<T>{}, table, gate);
         }
         launch_rx<T>(rd, out, tot[b ^ 1].as<T>(), zc, g, gate, RxAction{-1, 0, 0, -1, 0, 0}, stream);
@@ -1240,7 +1245,7 @@ template <typename T> struct SimImpl : SimBase {
     // ---- per-stage seam
     void upcontinuation() override {
         FieldSet<T> f = fs(cur);
-        launch_boundary<T>(bd, g, f.bz, tot[cur].as<T>(), zc.n, f.bx, f.by, StepGate{nullptr, 0, 0}, stream);
+        launch_boundary<T>(bd, g, f.bz, tot[cur].as<T>(), zc.n, f.bx, f.by, StepGate{nullptr, 0, 0}, stream, cols_alone);
         CK(cudaGetLastError());
     }
     // the same pipeline with its four work arrays carved from caller-provided scratch
@@ -1263,7 +1268,7 @@ template <typename T> struct SimImpl : SimBase {
         b2.VY = reinterpret_cast<C2<T> *>(p + off[2]);
         b2.Z = reinterpret_cast<C2<T> *>(p + off[3]);
         FieldSet<T> f = fs(cur);
-        launch_boundary<T>(b2, g, f.bz, tot[cur].as<T>(), zc.n, f.bx, f.by, StepGate{nullptr, 0, 0}, stream);
+        launch_boundary<T>(b2, g, f.bz, tot[cur].as<T>(), zc.n, f.bx, f.by, StepGate{nullptr, 0, 0}, stream, cols_alone);
         CK(cudaGetLastError());
     }
     StepScalars<T> scal(double lam, double dt, double dtb, double wave) {
@@ -1573,7 +1578,7 @@ template <typename T> struct SimImpl : SimBase {
             CK(cudaEventRecord(e0, stream));
             for (int r = 0; r < reps; r++) {
                 FieldSet<T> f = fs(r & 1);
-                launch_boundary<T>(bd, g, f.bz, tot[r & 1].as<T>(), zc.n, f.bx, f.by, StepGate{nullptr, 0, 0}, stream);
+                launch_boundary<T>(bd, g, f.bz, tot[r & 1].as<T>(), zc.n, f.bx, f.by, StepGate{nullptr, 0, 0}, stream, cols_alone);
             }
             CK(cudaEventRecord(e1, stream));
             CK(cudaEventSynchronize(e1));
