@@ -46,6 +46,8 @@ template <typename T> __global__ void k_bilinear(BoundaryDev<T> bd, T *bx, T *by
 }
 
 // ---- batched kernels: block b works for slot idx.slot_of(b)
+// (FP32: six blocks on an SM, 40 registers.  With 46 it was five, and 8 surveys of up to 64 x 64 x 48 took 56.3 us per step
+// instead of 49.7; the others measured, 4 to 8 of up to 200 x 180 x 120, take the same.)
 template <typename T>
 __device__ __forceinline__ const BoundarySlot<T> *bnd_slot(const BoundarySlot<T> *slots, const BatchIndex &idx,
                                                            int s, int &lb) {
@@ -56,14 +58,14 @@ __device__ __forceinline__ const BoundarySlot<T> *bnd_slot(const BoundarySlot<T>
     return d;
 }
 template <typename T>
-__global__ void __launch_bounds__(kBndThreads)
+__global__ void __launch_bounds__(kBndThreads, sizeof(T) == 4 ? 6 : 4)
     k_rows_fwd_b(const BoundarySlot<T> *__restrict__ slots, const __grid_constant__ BatchIndex idx, int s) {
     int lb;
     const BoundarySlot<T> *d = bnd_slot(slots, idx, s, lb);
     if (d) rows_fwd_cta<T>(d->bd, d->bz, d->tot, d->nch, d->g, lb);
 }
 template <typename T>
-__global__ void __launch_bounds__(kBndThreads)
+__global__ void __launch_bounds__(kBndThreads, sizeof(T) == 4 ? 6 : 4)
     k_cols_b(const BoundarySlot<T> *__restrict__ slots, const __grid_constant__ BatchIndex idx, int s) {
     int lb;
     const BoundarySlot<T> *d = bnd_slot(slots, idx, s, lb);
