@@ -398,7 +398,8 @@ def run_gb300(args, dist):
     ms_max = dist.reduce(ms, "max")
     work = dist.reduce(cells * K, "sum")
     value = work / (ms_max * 1e-3) / 1e9
-    launches = K * sim.info["launches_per_step"] + math.ceil(K / gsteps)
+    per_step = sim.info["launches_per_step"]  # 0: cooperative launches of up to 512 steps
+    launches = K * per_step + math.ceil(K / (gsteps if per_step else 512))
     # per-kernel timings on the same stream (events around standalone launches)
     _, ms_sweep, ms_bnd = sim.time_steps(0, 64)
     sim.close()
