@@ -176,7 +176,7 @@ template <typename T> struct BatchImpl : BatchBase {
     // 2 surveys of 44 x 38 x 27 (10) 45, 35, 34, 45; 8 of up to 64 x 64 x 48 (52) 65, 70, 57, 67; 2 of 128 x 128 x 96 (62)
     // 110, 116, 95, 108; 6 of 95 x 67 x 39 (90) 69, 59, 53, 72; 6 of 119 x 83 x 43 (114) 95, 75, 94, 91; 4 of
     // 145 x 117 x 61 (150) 115, 93, 93, 109; 8 of 152 x 131 x 112 (300) 196, 195, -, 175; 4 of 200 x 180 x 120 (330) 206, 202,
-    // -, 185.
+    // -, 185.  (With five blocks of the boundary's kernels on an SM; with six the 8 of up to 64 x 64 x 48 take 50, spread.)
     void plan_step() {
         const int n = (int)running.size();
         bool whole = !persistent && n > 0;

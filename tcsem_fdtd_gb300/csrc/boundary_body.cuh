@@ -125,7 +125,8 @@ template <typename T> __host__ __device__ inline ColsLayout cols_layout(const Bo
     // The remap's tables, its column and its spline moments lie where the transforms come later: behind the M1
     // points that the remap writes.  A column of a 736-point plane needs 35 KB instead of 55, so three blocks
     // instead of two run beside a sweep CTA (256 x 256 x 160, whose step waits for them: 132.4 -> 129.4 us with the
-    // packed sums of fft.cuh; FP64, the boundary alone: 170 -> 160 us).
+    // packed sums of fft.cuh; FP64, the boundary alone: 170 -> 161 us).  Where more of them on an SM is worse, the
+    // launch asks for more (cols_apart, cols_even).
     size_t p = l.a + rnd16(bd.M1 * sizeof(C2<T>));
     l.tab = p; p += rnd16(bd.ry.nT * sizeof(T));
     l.tabi = p; p += rnd16(bd.ry.nI * sizeof(int));

@@ -161,11 +161,11 @@ struct BatchIndex {
     }
 };
 
-// everything one step of the fused sweep needs for one slot (device memory)
 // A launch may take a chunk in two: all but its top plane, and after that the top plane, whose Bz goes on from the
 // plane below it (the same sums in the same order as the whole chunk's)
 enum class Piece { WHOLE, LOWER, TOP };
 
+// everything one step of the fused sweep needs for one slot (device memory)
 template <typename T> struct SweepSlot {
     SweepMaps maps;
     Geom g;

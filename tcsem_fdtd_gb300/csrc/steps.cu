@@ -14,7 +14,7 @@
 //     reads the field set step s wrote.
 // What bounds it: the chain boundary -> top plane -> barrier, and where a chunk is deep the march of its planes
 // (0.8 us each with one CTA on an SM).  64 x 64 x 48 with a 260 x 260 plane, us per step: about 3 from the barrier to
-// the columns of F, 4 through y, 4 to the air plane, 4.5 for the top plane, 1.3 for the barrier; 19.2 in all, 25.8
+// the columns of F, 4 through y, 4 to the air plane, 4.5 for the top plane, 1.3 for the barrier; 18.9 in all, 25.8
 // as a captured graph, whose four boundary kernels alone take 20.7.
 // Every wait is bounded in time: a CTA that gives up sets the abort flag and the error word, and every
 // CTA leaves at its next wait.

@@ -123,6 +123,8 @@ template <bool FRESH> __device__ __forceinline__ Vec4<float> ld4(const float *p)
 // product's) shares are added as a tree.  Relative error of the air plane, geometric mean over 16 grids
 // and three fields each: transforms in FP32 1.67e-7; whole chains, shares added one after the other 1.75e-7; as a
 // tree 1.60e-7; put aside too 1.54e-7 (0.1 to 0.5 us per step).  Two chains side by side in a warp take 1 to 1.6 us.
+// Of whole runs the errors are the same: traces of 22 surveys (470 to 1860 steps) against FP64, this form over the
+// transforms, 0.23 to 1.9 in single ones; geometric mean 0.98 of the rms error and 1.00 of the largest.
 
 // ---- first and third product: Out[j][n] = sum_k X[j][k] Tab[k][n], one tile of J j by 32 n per CTA.
 // The table's block streams through shared memory by bulk copies that are issued before the CTA waits for

@@ -30,10 +30,10 @@ namespace tcsem {
 //                 ->  Bz(k+1)
 //
 // What bounds it: memory.  256 x 256 x 160 in FP32 (545 MB of algorithmic traffic, 80 us at the copy rate)
-// takes 111.1 us, with DRAM busy 69 % of the time and issue slots 40 %; with register stores, scalar
-// arithmetic and two iterations of lead for the copies it was 119.3 us and 74 instead of 49 million
-// warp-instructions.  The pieces, measured one after the other: TMA stores and packed arithmetic 115.8 us
-// (and 17 -> 14.5 us on 64 x 64 x 48, which stays in L2), the third iteration of lead 111.1 us.
+// takes 110 to 112 us, with DRAM busy 67 % of the time, issue slots 43 % and 51 million warp-instructions; with
+// register stores, scalar arithmetic and two iterations of lead for the copies it was 119 us and 74 million.
+// The pieces, measured one after the other: TMA stores and packed arithmetic 115.8 us (and 17 -> 14.5 us on
+// 64 x 64 x 48, which stays in L2), the third iteration of lead 111.1 us.
 //
 // Bz within a chunk is the partial sum P(k) = sum_{k'=k}^{k1-1} dz div_xy B(k');
 // the true Bz(k) = P(k) + O_c with O_c = sum of the chunk totals T_c' of the
