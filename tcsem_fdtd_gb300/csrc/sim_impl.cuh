@@ -368,7 +368,9 @@ template <typename T> struct SimImpl : SimBase {
         // 60.5; 1.1 (three grids) 52.4, 61.0, 66.7 and 51.7, 59.5, 65.5; 1.3 (four) 53.2, 72.1, 49.8, 65.8 and 50.4, 65.4, 52.1, 68.7;
         // 1.4 (180 x 180 x 60) 59.8 and 57.0; 1.6 (128 x 160 x 110) 69.8 and 73.0; 1.8 to 2.2 (five) 56.5, 66.3, 81.0, 77.1, 116.9 and
         // 52.8, 62.7, 70.5, 70.4, 95.2; 2.9 97.2 and 92.3; 5.9 142.7 and 133.  Planes of up to 430 points: no difference.
-        if (t_bnd > t_sweep) cols_beside = cols_apart(bd);
+        // In FP64 blocks in flight count for more: by the same ratio 1.0 (three) 184.8, 173.0, 850 and 199.0, 155.2, 848; 1.2 391
+        // and 414; 1.5 313 and 335; 15 1246 and 1319.
+        if (sizeof(T) == 4 && t_bnd > t_sweep) cols_beside = cols_apart(bd);
         zero_state();
     }
 
